@@ -100,7 +100,7 @@ def draw(rng):
                     marangoni=rng.random() < 0.5, check=rng.choice([0, 50, 100]))
     if kind == "foam":
         return {"kind": kind, "bubbles": _log(rng, 12, 300), "steps": rng.randint(50, 400), "rmin": 32,
-                "rmax": rng.choice([128, 256, 512]), "step": rng.choice([1, 2, 32])}
+                "rmax": rng.choice([128, 256, 512]), "step": rng.choice([2, 2, 32])}
     if kind == "spectral":
         return {"kind": kind, "n": _log(rng, 10_000, 4_000_000), "nl": rng.choice([81, 81, 41, 16, 128]),
                 "mode": rng.choice(["tc", "fp32"])}
