@@ -263,8 +263,9 @@ int sbs_gpu_drainage_set_marangoni_params(sbs_drainage *h, float gamma_air, floa
                                           float surfactant_diffusion, float marangoni_coeff);
 /* Steps advanced per kernel launch (no reference counterpart). 2..4 use the
  * temporally blocked kernel (one read and one write of the fields per K steps;
- * grid_width must be a multiple of 4), 0 or 1 launch one step at a time. The
- * results are bit-identical either way. Default 4 where supported. */
+ * choosing K needs a grid_width that is a multiple of 4), 0 or 1 launch one step
+ * at a time. The results are bit-identical either way. Default 4; other widths
+ * (at least 8) are blocked by default too, which time_blocking reports as 1. */
 int sbs_gpu_drainage_set_time_blocking(sbs_drainage *h, int steps_per_launch);
 int sbs_gpu_drainage_time_blocking(const sbs_drainage *h, int *out);
 /* The same for a handle of either semantics (no reference counterpart). For the
@@ -272,9 +273,10 @@ int sbs_gpu_drainage_time_blocking(const sbs_drainage *h, int *out);
  * pole-ring means and the marginal-regeneration fronts K steps at a time (row
  * strips of blocks spanning the ring, all resident at once; the two polar
  * strips meet at a bounded barrier per ring mean, see sbs_set_wait_limit); it
- * needs an even resolution and at least 2 (K + 1) theta rows. Results are
- * bit-identical to single steps. Default where supported: 3 for the
- * compensated f32x2 storage, 4 for plain f32 (WGSL semantics: 4). */
+ * needs at least 2 (K + 1) theta rows, and choosing K an even resolution. Results
+ * are bit-identical to single steps. Default where supported: 3 for the
+ * compensated f32x2 storage, 4 for plain f32 (WGSL semantics: 4); odd resolutions
+ * are blocked by default too, which time_blocking() reports as 1. */
 int sbs_drainage_set_time_blocking(sbs_drainage *h, int steps_per_launch);
 int sbs_drainage_time_blocking(const sbs_drainage *h, int *out);
 

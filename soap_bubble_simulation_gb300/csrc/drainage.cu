@@ -259,21 +259,20 @@ int allocate(sbs_drainage *h) {
             const StepGeom g = wtb_geometry(h->nt, h->np, k);
             vol_blocks = std::max(vol_blocks, (size_t)g.nbx * g.nby);
         }
-    if (h->sem == SBS_CPU_SEMANTICS) {
-        size_t parts = 1;
+    size_t slots = 0;
+    if (h->sem == SBS_CPU_SEMANTICS)
         for (int k = 2; k <= 4; ++k) {
             const StepGeom g = wtbc_geometry(h->nt, h->np, k, h->x2);
             vol_blocks = std::max(vol_blocks, (size_t)g.nbx * g.nby);
-            parts = std::max(parts, (size_t)wtbc_ring_parts(g));
+            slots = std::max(slots, wtbc_ring_bytes(g));
         }
-        SBS_CUDA_TRY(cudaMalloc(&h->ring_part, sizeof(FixSum) * 2 * 4 * parts));
-        SBS_CUDA_TRY(cudaMalloc(&h->ring_bar, sizeof(unsigned) * kWtbcBarWords));
-        SBS_CUDA_TRY(cudaMemset(h->ring_bar, 0, sizeof(unsigned) * kWtbcBarWords));
-        SBS_CUDA_TRY(cudaHostAlloc(&h->ring_status, sizeof(unsigned), cudaHostAllocMapped));
-        *h->ring_status = 0u;
-        SBS_CUDA_TRY(cudaHostGetDevicePointer(&h->ring_status_dev, h->ring_status, 0));
-        h->wait_epoch = wait_config().epoch;
-    }
+    h->ring_bytes = slots + sizeof(unsigned long long);
+    SBS_CUDA_TRY(cudaMalloc(&h->ring_slots, h->ring_bytes));
+    SBS_CUDA_TRY(cudaMemset(h->ring_slots, 0, h->ring_bytes));
+    SBS_CUDA_TRY(cudaHostAlloc(&h->ring_status, sizeof(unsigned), cudaHostAllocMapped));
+    *h->ring_status = 0u;
+    SBS_CUDA_TRY(cudaHostGetDevicePointer(&h->ring_status_dev, h->ring_status, 0));
+    h->wait_epoch = wait_config().epoch;
     SBS_CUDA_TRY(cudaMalloc(&h->vol_partials, sizeof(double) * vol_blocks));
     SBS_CUDA_TRY(cudaMalloc(&h->vol_counter, sizeof(unsigned) * 2));
     SBS_CUDA_TRY(cudaMemset(h->vol_counter, 0, sizeof(unsigned) * 2));
@@ -314,19 +313,34 @@ void release(sbs_drainage *h) {
     cudaFree(h->red_out);
     cudaFree(h->sched_dev);
     cudaFree(h->qbuf);
-    cudaFree(h->ring_part);
-    cudaFree(h->ring_bar);
+    cudaFree(h->ring_slots);
     cudaFree(h->cau_buf);
     if (h->ring_status) cudaFreeHost(h->ring_status);
     if (h->stream) cudaStreamDestroy(h->stream);
 }
 
+// Grids whose rows are no multiple of four cells are blocked by default like all others, but their
+// blocking is not a setting: set_time_blocking() refuses to choose a K for them (it can turn
+// blocking off) and time_blocking() reports 1.
+bool blocking_selectable(const sbs_drainage *h) { return h->np % 4 == 0; }
+
 // Whether a chunk of `count` WGSL passes ends with the launch that also writes the caustic map:
 // the final chunk of a run that asked for the map, blocked, with three passes before the final
 // single pass (the map is of the field one pass behind the newest, the buffer the renderer binds).
 bool cau_plan(const sbs_drainage *h, int count, bool last_single) {
-    return h->cau_on && h->sem == SBS_WGSL_SEMANTICS && h->wtb_k > 1 && last_single && h->cau_geom.nby > 0 &&
-           count - 1 >= kWtbCausticK;
+    return h->cau_on && h->sem == SBS_WGSL_SEMANTICS && h->wtb_k > 1 && last_single &&
+           h->cau_geom.nby > 0 && count - 1 >= kWtbCausticK;
+}
+
+// The bounded waits' limit and status words, the test switch that makes them run out, and the ring's
+// reciprocal length.
+void wait_args(sbs_drainage *h, StepArgs *a) {
+    const WaitConfig wc = wait_config();
+    a->ring_status = reinterpret_cast<unsigned *>(h->ring_slots + h->ring_bytes / sizeof(*h->ring_slots) - 1);
+    a->status_host = h->ring_status_dev;
+    a->wait_cycles = wc.cycles;
+    a->extra = (wc.stall & SBS_STALL_GRID_BARRIER) ? 1u : 0u;
+    a->inv_np = 1.0 / (double)h->np;
 }
 
 // Enqueues `count` steps starting from buffer `start`; returns the buffer holding the result.
@@ -375,15 +389,8 @@ int enqueue_steps(sbs_drainage *h, int start, int count, float dt, bool vol_last
             a.b = k.b;
             a.DR2 = k.DR2;
             a.dt = dt;
-            a.prow = h->cgeom.prow;
-            a.ring_part = h->ring_part;
-            a.ring_bar = h->ring_bar;
-            a.status_host = h->ring_status_dev;
-            {
-                const WaitConfig wc = wait_config();
-                a.wait_cycles = wc.cycles;
-                a.extra = (wc.stall & SBS_STALL_GRID_BARRIER) ? 1u : 0u;
-            }
+            a.ring_slots = h->ring_slots;
+            wait_args(h, &a);
             if (blocked)
                 SBS_CUDA_TRY(launch_wtbc(K, h->x2, a, h->cgeom, h->stream));
             else
@@ -483,22 +490,25 @@ int launches_in(const sbs_drainage *h, int count, bool last_single) {
 // Runs one chunk (count <= kMaxChunk) through a cached CUDA graph (or directly when short).
 int run_chunk(sbs_drainage *h, int count, double dt, bool vol_last, bool last_single) {
     const bool cpu = h->sem == SBS_CPU_SEMANTICS;
-    const bool use_sched = cpu && h->tfe.enabled;
+    bool use_sched = false;  // some step of the chunk has a front
     float dtf;
     if (cpu) {
         dtf = (float)dt;
-        if (use_sched) {
+        if (h->tfe.enabled) {
             const int slot = h->sched_slot;
             SBS_CUDA_TRY(cudaEventSynchronize(h->sched_ev[slot]));
             TfeStep *hs = h->sched_host[slot];
             for (int i = 0; i < count; ++i) {
                 h->tfe.advance(h->current_time, dt, h->nt, h->np, hs + i);
                 h->current_time += dt;
+                use_sched = use_sched || hs[i].nf > 0;
             }
-            SBS_CUDA_TRY(cudaMemcpyAsync(h->sched_dev, hs, sizeof(TfeStep) * count, cudaMemcpyHostToDevice,
-                                         h->stream));
-            SBS_CUDA_TRY(cudaEventRecord(h->sched_ev[slot], h->stream));
-            h->sched_slot ^= 1;
+            if (use_sched) {  // else the steps run without a schedule, in kernels without the fronts' code
+                SBS_CUDA_TRY(cudaMemcpyAsync(h->sched_dev, hs, sizeof(TfeStep) * count, cudaMemcpyHostToDevice,
+                                             h->stream));
+                SBS_CUDA_TRY(cudaEventRecord(h->sched_ev[slot], h->stream));
+                h->sched_slot ^= 1;
+            }
         } else {
             for (int i = 0; i < count; ++i) h->current_time += dt;
         }
@@ -551,20 +561,20 @@ int run_chunk(sbs_drainage *h, int count, double dt, bool vol_last, bool last_si
     return SBS_OK;
 }
 
-// After the stream has drained: a timed-out ring barrier of the blocked CPU-semantics step turns
-// into SBS_E_TIMEOUT, and the barrier words are cleared for the next call.
+// After the stream has drained: a timed-out ring exchange of the blocked CPU-semantics step turns
+// into SBS_E_TIMEOUT, and its slots (whose tags count on) and the status are cleared for the next call.
 int check_ring_status(sbs_drainage *h) {
     if (!h->ring_status || *(volatile unsigned *)h->ring_status == 0u) return SBS_OK;
     *(volatile unsigned *)h->ring_status = 0u;
-    SBS_CUDA_TRY(cudaMemsetAsync(h->ring_bar, 0, sizeof(unsigned) * kWtbcBarWords, h->stream));
+    SBS_CUDA_TRY(cudaMemsetAsync(h->ring_slots, 0, h->ring_bytes, h->stream));
     SBS_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    return set_error(SBS_E_TIMEOUT, "drainage: a pole-ring barrier wait timed out");
+    return set_error(SBS_E_TIMEOUT, "drainage: a wait for another block's ring sum timed out");
 }
 
 // Advances n steps in chunks; a volume check follows every check_every-th step (0 = none).
 int run_steps(sbs_drainage *h, double dt, uint64_t n, uint32_t check_every) {
     if (h->tfe.error) return set_error(SBS_E_STATE, "TFE front columns are not one interval");
-    if (h->ring_bar) {
+    if (h->ring_slots) {
         const unsigned epoch = wait_config().epoch;
         if (epoch != h->wait_epoch) {  // the launches carry the wait settings: capture them again
             SBS_CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -618,7 +628,7 @@ int run_with_caustics(sbs_drainage *h, uint32_t passes, const sbs_caustic_params
     }
     if (mem == SBS_MEM_HOST) SBS_CUDA_TRY(cudaMemcpyAsync(map, dst, bytes, cudaMemcpyDeviceToHost, h->stream));
     SBS_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    return SBS_OK;
+    return check_ring_status(h);
 }
 
 int field_reduce(sbs_drainage *h, ReduceOut *out) {
@@ -825,7 +835,7 @@ int sbs_gpu_drainage_step(sbs_drainage *h, float frame_dt) {
     h->current_time = t0;
     for (uint32_t i = 0; i < h->steps_per_frame; ++i) h->current_time += (double)step_dt;
     SBS_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    return SBS_OK;
+    return check_ring_status(h);
 }
 
 int sbs_gpu_drainage_run(sbs_drainage *h, uint32_t passes) {
@@ -835,7 +845,7 @@ int sbs_gpu_drainage_run(sbs_drainage *h, uint32_t passes) {
     int rc = run_steps(h, 0.0, passes, 0);
     if (rc) return rc;
     SBS_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    return SBS_OK;
+    return check_ring_status(h);
 }
 
 int sbs_gpu_drainage_run_caustics(sbs_drainage *h, uint32_t passes, const sbs_caustic_params *p, float *caustic_map,
@@ -1191,7 +1201,7 @@ int sbs_gpu_drainage_set_time_blocking(sbs_drainage *h, int steps_per_launch) {
     CHECK_HANDLE(h);
     REQUIRE_SEM(h, SBS_WGSL_SEMANTICS);
     SBS_CHECK_ARG(steps_per_launch >= 0 && steps_per_launch <= 4, "steps_per_launch must be 0..4");
-    if (steps_per_launch > 1 && !wtb_supported(h->nt, h->np))
+    if (steps_per_launch > 1 && !(blocking_selectable(h) && wtb_supported(h->nt, h->np)))
         return set_error(SBS_E_INVALID, "time blocking needs grid_width a multiple of 4 (got %d)", h->np);
     destroy_graphs(h);
     h->wtb_k = steps_per_launch > 1 ? steps_per_launch : 0;
@@ -1202,7 +1212,7 @@ int sbs_gpu_drainage_set_time_blocking(sbs_drainage *h, int steps_per_launch) {
 int sbs_gpu_drainage_time_blocking(const sbs_drainage *h, int *out) {
     CHECK_HANDLE(h);
     SBS_CHECK_ARG(out != nullptr, "out is null");
-    *out = h->wtb_k > 1 ? h->wtb_k : 1;
+    *out = blocking_selectable(h) && h->wtb_k > 1 ? h->wtb_k : 1;
     return SBS_OK;
 }
 
@@ -1213,7 +1223,7 @@ int sbs_drainage_set_time_blocking(sbs_drainage *h, int steps_per_launch) {
     SBS_CHECK_ARG(steps_per_launch >= 0 && steps_per_launch <= 4, "steps_per_launch must be 0..4");
     StepGeom g{};
     if (steps_per_launch > 1) {
-        g = wtbc_geometry(h->nt, h->np, steps_per_launch, h->x2);
+        if (blocking_selectable(h)) g = wtbc_geometry(h->nt, h->np, steps_per_launch, h->x2);
         if (g.nby < 1)
             return set_error(SBS_E_INVALID,
                              "time blocking needs an even resolution and at least %d theta rows (grid %d x %d)",
@@ -1230,7 +1240,7 @@ int sbs_drainage_time_blocking(const sbs_drainage *h, int *out) {
     CHECK_HANDLE(h);
     SBS_CHECK_ARG(out != nullptr, "out is null");
     if (h->sem == SBS_WGSL_SEMANTICS) return sbs_gpu_drainage_time_blocking(h, out);
-    *out = h->cpu_k > 1 ? h->cpu_k : 1;
+    *out = blocking_selectable(h) && h->cpu_k > 1 ? h->cpu_k : 1;
     return SBS_OK;
 }
 

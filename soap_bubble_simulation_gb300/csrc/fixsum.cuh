@@ -185,6 +185,117 @@ __device__ __forceinline__ FixSum fix_ldcg(const FixSum *p) {
     v.pad = 0u;
     return v;
 }
+
+// The same sums for the words of every film that has not blown up, or thinned to nothing: thickness
+// words that are 0 or in [2^-47, 2^-16) m (7e-15 m .. 15 um) and low words of at most 2^-41 m. The
+// first are whole numbers of 2^-70 m below 2^54, the second, truncated, whole numbers of 2^-96 m up
+// to 2^55; 128 of either (a warp's) fit 64 bits, so a word costs a multiplication, a conversion and
+// an addition, against ~60 emulated 64-bit operations, and a warp's total six REDUX instead of 45
+// shuffles. Partials travel as the 128-bit total, the low half of the 256-bit one.
+struct Fix128 {
+    unsigned w0, w1, w2, w3;  // two's complement, little-endian words
+};
+
+__device__ __forceinline__ void fix128_add_words(Fix128 &a, unsigned b0, unsigned b1, unsigned b2, unsigned b3) {
+    asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, %5;\n\taddc.cc.u32 %2, %2, %6;\n\taddc.u32 %3, %3, %7;"
+        : "+&r"(a.w0), "+&r"(a.w1), "+&r"(a.w2), "+r"(a.w3)
+        : "r"(b0), "r"(b1), "r"(b2), "r"(b3));
+}
+
+// The warp's total in every lane: 27-bit pieces, whose sums over 32 lanes fit 32 bits.
+__device__ __forceinline__ Fix128 fix128_warp(const Fix128 &a) {
+    constexpr unsigned kM = (1u << 27) - 1u;
+    const unsigned s0 = __reduce_add_sync(0xffffffffu, a.w0 & kM);
+    const unsigned s1 = __reduce_add_sync(0xffffffffu, __funnelshift_r(a.w0, a.w1, 27) & kM);
+    const unsigned s2 = __reduce_add_sync(0xffffffffu, __funnelshift_r(a.w1, a.w2, 22) & kM);
+    const unsigned s3 = __reduce_add_sync(0xffffffffu, __funnelshift_r(a.w2, a.w3, 17) & kM);
+    const unsigned s4 = __reduce_add_sync(0xffffffffu, a.w3 >> 12);
+    Fix128 t{s0, 0u, 0u, 0u};
+    fix128_add_words(t, s1 << 27, s1 >> 5, 0u, 0u);
+    fix128_add_words(t, 0u, s2 << 22, s2 >> 10, 0u);
+    fix128_add_words(t, 0u, 0u, s3 << 17, s3 >> 15);
+    t.w3 += s4 << 12;
+    return t;
+}
+
+__device__ __forceinline__ unsigned long long fix64_warp(unsigned long long x) {
+    constexpr unsigned kM = (1u << 27) - 1u;
+    const unsigned s0 = __reduce_add_sync(0xffffffffu, (unsigned)x & kM);
+    const unsigned s1 = __reduce_add_sync(0xffffffffu, (unsigned)(x >> 27) & kM);
+    const unsigned s2 = __reduce_add_sync(0xffffffffu, (unsigned)(x >> 54));
+    return s0 + ((unsigned long long)s1 << 27) + ((unsigned long long)s2 << 54);
+}
+
+// Whether the first nv of a lane's four thickness words and low words are in the range above.
+template <bool X2>
+__device__ __forceinline__ bool fix128_takes(const float (&h)[4], const float (&l)[4], int nv) {
+    constexpr unsigned kLow = (127u - 47u) << 23, kHigh = (127u - 16u) << 23, kLo = (127u - 41u) << 23;
+    unsigned top = 0u, bottom = 0xffffffffu, lo = 0u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const unsigned u = __float_as_uint(k < nv ? h[k] : 0.f);
+        top = max(top, u);
+        bottom = min(bottom, u - 1u);  // 0 wraps to the largest
+        if (X2) lo = max(lo, __float_as_uint(k < nv ? l[k] : 0.f) & 0x7fffffffu);
+    }
+    return top < kHigh && bottom >= kLow - 1u && lo <= kLo;
+}
+
+// The warp's total of such words, in every lane.
+template <bool X2>
+__device__ __forceinline__ Fix128 fix128_sum(const float (&h)[4], const float (&l)[4], int nv) {
+    long long H = 0, L = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        H += __float2ll_rz((k < nv ? h[k] : 0.f) * 0x1p70f);
+        if (X2) L += __float2ll_rz((k < nv ? l[k] : 0.f) * 0x1p96f);
+    }
+    const unsigned long long th = fix64_warp((unsigned long long)H);
+    const long long tl = X2 ? (long long)fix64_warp((unsigned long long)L) : 0;
+    Fix128 t{(unsigned)(th << 26), (unsigned)(th >> 6), (unsigned)(th >> 38), 0u};
+    const unsigned sign = (unsigned)(tl >> 63);
+    if (X2) fix128_add_words(t, (unsigned)tl, (unsigned)((unsigned long long)tl >> 32), sign, sign);
+    return t;
+}
+
+// fix_to_double of the sign-extended total (below 2^127 in magnitude).
+__device__ __forceinline__ double fix128_to_double(const Fix128 &a) {
+    unsigned long long lo = ((unsigned long long)a.w1 << 32) | a.w0, hi = ((unsigned long long)a.w3 << 32) | a.w2;
+    const bool neg = (hi >> 63) != 0ull;
+    if (neg) {
+        lo = ~lo + 1ull;
+        hi = ~hi + (lo == 0ull ? 1ull : 0ull);
+    }
+    unsigned long long top = lo;
+    int scale = -kFixShift;
+    if (hi) {  // the top 64 bits plus a sticky bit for everything below them
+        const int lz = __clzll((long long)hi);
+        top = lz ? (hi << lz) | (lo >> (64 - lz)) : hi;
+        top |= (lo << lz) != 0ull ? 1ull : 0ull;
+        scale += 64 - lz;
+    }
+    if (top == 0ull) return 0.0;
+    // times 2^scale: the exponent stays far inside the normal range
+    const double d = __longlong_as_double(__double_as_longlong((double)top) + ((long long)scale << 52));
+    return neg ? -d : d;
+}
+
+// The ring's mean, sum / n rounded once, as the f32 pair (hi, lo). inv = 1 / n rounded: with it the
+// quotient takes three FP64 operations (q = a y, then q + (a - q n) y; Markstein, IBM J. Res. Dev.
+// 34, 1990, theorem 1: exact rounding from a rounded reciprocal) instead of a division's ~30, at
+// 1/64 of the FP32 rate.
+template <bool X2>
+__device__ __forceinline__ float2 fix_mean(double sum, double n, double inv) {
+    const double q = sum * inv;
+    const double m = fma(fma(-q, n, sum), inv, q);
+    const float mh = (float)m;
+    return make_float2(mh, X2 ? (float)(m - (double)mh) : 0.f);
+}
+
+__device__ __forceinline__ FixSum fix_widen(const Fix128 &a) {
+    const unsigned long long top = (a.w3 >> 31) ? ~0ull : 0ull;
+    return FixSum{((unsigned long long)a.w1 << 32) | a.w0, ((unsigned long long)a.w3 << 32) | a.w2, top, top, 0u, 0u};
+}
 #endif
 
 }  // namespace sbs

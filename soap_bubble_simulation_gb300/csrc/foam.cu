@@ -85,80 +85,52 @@ __device__ bool grid_barrier(unsigned *bar, unsigned nblocks, unsigned extra, lo
 // cell-steps/s against 5.35e11; four blocks (128 registers) 4.98e11.
 constexpr int kMinBlocksPerSm = 3;
 
-template <int K, bool MAR>
+template <int K, bool MAR, bool RAG>
 __global__ void __launch_bounds__(kWarps * 32, kMinBlocksPerSm) foam_kernel(const FoamArgs a) {
-    extern __shared__ float4 s_co_all[];  // per warp: rbmax + 2K coefficient rows
+    extern __shared__ float4 s_dyn[];  // per warp: its row ring, the coefficients of rbmax + 2K rows
     __shared__ int s_timeout;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gw = blockIdx.x * kWarps + warp, nw = gridDim.x * kWarps;
-    float4 *s_co = s_co_all + warp * (a.rbmax + 2 * K);
+    float4 *s_ring = s_dyn + warp * (kWtbRingBytes / sizeof(float4) + 2 * (a.rbmax + 2 * K));
+    float4 *s_co = s_ring + kWtbRingBytes / sizeof(float4);
 
     for (int ph = 0; ph < a.nphases; ++ph) {
         const int par = (a.parity0 + ph) & 1;
         for (int it = gw; it < a.nitems; it += nw) {
             const FoamItem item = a.items[it];
             const FoamBubble &B = a.bubbles[item.bubble];
-            const int nt = B.nt, np = B.np;
             __syncwarp();
-            for (int i = lane; i < item.r1 - item.r0 + 2 * K; i += 32) {
-                const int r = item.r0 - K + i;
-                s_co[i] = (r >= 0 && r < nt) ? __ldg(B.rows + r) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+            for (int i = lane; i < item.r1 - item.r0 + 2 * K; i += 32)
+                wtb_coefficients(s_co, i, B.rows, item.r0 - K + i, B.nt);
             __syncwarp();
-            const int out0 = item.seg * kSeg;
-            const int cu = out0 - 4 + 4 * lane;
-            const int col = ((cu % np) + np) % np;
-            Wtb w;
-            w.hin = B.h[par] + col;
-            w.cin = B.c[par] + col;
-            w.hout = B.h[par ^ 1] + col;
-            w.cout = B.c[par ^ 1] + col;
+            const int cu = item.seg * kSeg - 4 + 4 * lane;
+            Wtb<RAG> w{B.h[par], B.c[par], B.h[par ^ 1], B.c[par ^ 1], Cols<RAG>(cu, B.np), s_ring + lane};
             w.sco = s_co;
             w.sco_base = item.r0 - K;
-            w.nt = nt;
+            w.nt = B.nt;
             w.pitch = B.pitch;
             w.r0 = item.r0;
             w.r1 = item.r1;
-            w.store = lane >= 1 && lane <= 30 && cu < np;
-            w.b = B.b;
-            w.DR2 = B.DR2;
-            w.DsR2 = B.DsR2;
-            w.Gt = B.Gt;
-            w.M = B.M;
-            w.dt = a.dt;
-            w.crit = a.crit;
+            w.store = lane >= 1 && lane <= 30 && cu < B.np;
+            w.k = WgslK{B.b, B.DR2, B.DsR2, B.Gt, B.M, a.dt, a.crit};
             w.vol_w = nullptr;
-            float4 wh[K][3], wc[K][3];
-#pragma unroll
-            for (int l = 0; l < K; ++l)
-#pragma unroll
-                for (int s = 0; s < 3; ++s) {
-                    wh[l][s] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    wc[l][s] = wh[l][s];
-                }
             double vacc = 0.0;
-            const int t0 = w.r0 - K, t1 = w.r1 + K;
-            float4 ph4 = make_float4(0.f, 0.f, 0.f, 0.f), pc4 = ph4;
-            if (SBS_WTB_PREFETCH && t0 >= 0) {
-                ph4 = __ldcg(reinterpret_cast<const float4 *>(w.hin + (size_t)t0 * w.pitch));
-                pc4 = __ldcg(reinterpret_cast<const float4 *>(w.cin + (size_t)t0 * w.pitch));
-            }
-            for (int t = t0; t < t1; t += 3) {
-                wtb_iter<K, 0, false, MAR, true>(w, t, wh, wc, ph4, pc4, vacc);
-                if (t + 1 < t1) wtb_iter<K, 1, false, MAR, true>(w, t + 1, wh, wc, ph4, pc4, vacc);
-                if (t + 2 < t1) wtb_iter<K, 2, false, MAR, true>(w, t + 2, wh, wc, ph4, pc4, vacc);
-            }
+            wtb_strip<K, false, MAR, true, false, RAG>(w, vacc);
         }
         if (ph + 1 < a.nphases && !grid_barrier(a.bar, gridDim.x, a.extra, a.wait_cycles, &s_timeout)) return;
     }
 }
 
-const void *foam_fn(int K, bool mar) {
-    if (K == 1) return mar ? (const void *)foam_kernel<1, true> : (const void *)foam_kernel<1, false>;
-    if (K == 2) return mar ? (const void *)foam_kernel<2, true> : (const void *)foam_kernel<2, false>;
-    if (K == 4) return mar ? (const void *)foam_kernel<4, true> : (const void *)foam_kernel<4, false>;
+template <bool RAG>
+const void *foam_pick(int K, bool mar) {
+    if (K == 1) return mar ? (const void *)foam_kernel<1, true, RAG> : (const void *)foam_kernel<1, false, RAG>;
+    if (K == 2) return mar ? (const void *)foam_kernel<2, true, RAG> : (const void *)foam_kernel<2, false, RAG>;
+    if (K == 4) return mar ? (const void *)foam_kernel<4, true, RAG> : (const void *)foam_kernel<4, false, RAG>;
     return nullptr;
 }
+
+// rag: some bubble's rows are no multiple of four cells (an odd resolution).
+const void *foam_fn(int K, bool mar, bool rag) { return rag ? foam_pick<true>(K, mar) : foam_pick<false>(K, mar); }
 
 }  // namespace
 }  // namespace sbs
@@ -171,6 +143,7 @@ struct sbs_foam {
     std::vector<size_t> off, roff;
     std::vector<float> radius;
     size_t field_floats = 0;
+    bool ragged = false;  // some resolution is odd
     float *arena = nullptr;  // h0 | h1 | c0 | c1
     float4 *rows = nullptr;
     FoamBubble *d_bubbles = nullptr;
@@ -227,11 +200,12 @@ int build_items(sbs_foam *f, int rb) {
 int launch_phases(sbs_foam *f, int k, int phases) {
     if (phases <= 0) return SBS_OK;
     const bool mar = f->params.marangoni_enabled != 0;
-    const void *fn = foam_fn(k, mar);
-    const size_t smem = sizeof(float4) * (size_t)kWarps * (f->rbmax + 2 * k);
+    const void *fn = foam_fn(k, mar, f->ragged);
+    const size_t smem = kWarps * (kWtbRingBytes + 2 * sizeof(float4) * (size_t)(f->rbmax + 2 * k));
     int dev = 0, sms = 148, per_sm = 0;
     SBS_CUDA_TRY(cudaGetDevice(&dev));
     SBS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    SBS_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));  // tall strips
     SBS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kWarps * 32, smem));
     if (per_sm < 1) return set_error(SBS_E_CUDA, "foam kernel does not fit on an SM");
     FoamArgs a{};
@@ -340,6 +314,7 @@ int sbs_foam_create(uint32_t nbubbles, const uint32_t *resolution, const float *
     size_t off = 0, roff = 0;
     for (uint32_t b = 0; b < nbubbles; ++b) {
         const int nt = (int)resolution[b], np = 2 * nt;
+        f->ragged = f->ragged || np % 4 != 0;
         f->nt.push_back(nt);
         f->np.push_back(np);
         f->pitch.push_back((np + 31) / 32 * 32);

@@ -102,13 +102,13 @@ struct StepArgs {
     int poles_virtual;  // 1: pole rows of hin are the means of pin, not memory
     int marangoni;
     float crit, b, DR2, DsR2, Gt, M, dt;
+    double inv_np;      // 1 / np (pole-ring means)
     // blocked CPU-semantics step only: the polar strips' ring exchange
-    FixSum *ring_part;      // [2][4][C W] warp partials of ring 1 / ring N-2 per step of the launch
-    unsigned *ring_bar;     // [2][4] barrier words (arrivals, generation), then the status word
-    unsigned *status_host;  // host-mapped status word (nonzero: a barrier wait timed out)
-    long long wait_cycles;  // barrier wait limit
+    unsigned long long *ring_slots;  // the blocks' ring partials, 32-bit words tagged per exchange
+    unsigned *ring_status;           // nonzero: an exchange wait timed out
+    unsigned *status_host;           // host-mapped copy of it
+    long long wait_cycles;           // exchange wait limit
     unsigned extra;         // arrivals beyond the strip's blocks (1 only in the timeout test)
-    int prow;               // rows of each polar strip (0: all strips even)
     // blocked WGSL step only: the caustic map of the launch's result (nullptr: none)
     float *cau_out;         // grid_width x grid_height floats, row stride np
     float cau_focal, cau_scale, cau_sharp, cau_branch;
@@ -119,7 +119,6 @@ struct StepGeom {
     int nbx;  // column blocks
     int nby;  // row strips
     int rb;   // rows of the tallest strip
-    int prow; // blocked CPU-semantics step: rows of each polar strip (0: all strips even)
 };
 
 StepGeom step_geometry(int nt, int np, int semantics, int x2);
@@ -133,11 +132,10 @@ constexpr int kWtbCausticK = 3;
 // Temporally blocked CPU-semantics step (K = 2..4 steps per launch, pole means and fronts
 // included), drainage_wtb_cpu.cu. Each row strip is nbx blocks of wx warps that span the ring;
 // nby strips of at most rb rows, all resident at once (cooperative launch). nby == 0: the grid
-// is not supported. The ring exchange needs 2 x 4 x wtbc_ring_parts(g) FixSum partials and
-// kWtbcBarWords barrier words (zeroed before first use and after a timeout).
-constexpr int kWtbcBarWords = 17;
+// is not supported. The ring exchange needs wtbc_ring_bytes(g) of slots and a status word, zeroed
+// before first use and after a timeout.
 StepGeom wtbc_geometry(int nt, int np, int K, int x2);
-int wtbc_ring_parts(const StepGeom &g);
+size_t wtbc_ring_bytes(const StepGeom &g);
 cudaError_t launch_wtbc(int K, int x2, const StepArgs &a, const StepGeom &g, cudaStream_t s);
 // x2: compensated f32x2 thickness (hi + lo words); CPU semantics only.
 cudaError_t launch_step(int semantics, int x2, const StepArgs &a, const StepGeom &g, cudaStream_t s);
@@ -244,8 +242,8 @@ struct sbs_drainage {
     sbs::StepGeom wgeom{};
     int cpu_k = 0;  // steps per temporally blocked launch (CPU semantics; 0 = single steps only)
     sbs::StepGeom cgeom{};
-    sbs::FixSum *ring_part = nullptr;  // the blocked step's ring exchange (CPU semantics)
-    unsigned *ring_bar = nullptr;
+    unsigned long long *ring_slots = nullptr;  // the blocked step's ring exchange (CPU semantics), then the
+    size_t ring_bytes = 0;                     // waits' status word in the last 8 of ring_bytes
     unsigned *ring_status = nullptr;   // host-mapped timeout word
     unsigned *ring_status_dev = nullptr;
     unsigned wait_epoch = 0;           // the wait settings the captured graphs were made with

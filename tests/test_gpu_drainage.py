@@ -515,3 +515,87 @@ def test_time_blocking_needs_width_multiple_of_4(sbs):
         set_blocking(sbs, sim, 4)
     set_blocking(sbs, sim, 1)
     sim.run(5)
+
+
+@pytest.mark.parametrize("marangoni", [0, 1])
+@pytest.mark.parametrize("W,H", [(9, 5), (11, 40), (119, 37), (121, 64), (122, 33), (243, 70), (1037, 131)])
+def test_ragged_widths_blocked_by_default_match_single_steps(sbs, orc, W, H, marangoni):
+    """Widths that are no multiple of four cells (the seam inside a lane's window, one and several
+    120-column segments, a window that wraps more than once) run blocked by default: the bits of
+    single steps and of the kernel-order oracle, volumes, and the fused caustic map."""
+    from soap_bubble_simulation_gb300 import synthetic
+
+    h = synthetic.smooth_modes(H, W, seed=W + H).astype(np.float32)
+    h[H // 3, : W // 4] = 25e-9  # a patch below the critical thickness
+    h[2 * H // 3, W // 2] = 1e-4  # a spike that is clamped at zero around it
+    c = synthetic.surfactant_noise(H, W, seed=H)
+    c[1, :3] = (0.0, 1.0, 0.5)
+    out = []
+    for single in (False, True):
+        sim = sbs.GPUDrainageSimulator(None, 500e-9, W, H)
+        if single:
+            set_blocking(sbs, sim, 1)
+        sim.set_thickness_array(h)
+        sim.set_concentration_array(c)
+        sim.set_marangoni_enabled(bool(marangoni))
+        vols = sim.run_checked(0.001, 22, 11)
+        cau = sim.run_caustic_map(9)
+        out.append((sim.thickness_array(), sim.concentration_array(), cau, vols))
+    for a, b in zip(out[0][:3], out[1][:3]):
+        np.testing.assert_array_equal(a, b)
+    np.testing.assert_allclose(out[0][3], out[1][3], rtol=1e-12)
+    p = orc.wgsl_params(grid_width=W, grid_height=H, marangoni_enabled=marangoni)
+    ho, co = orc.wgsl_run(p, h, c, 31, "kernel")
+    np.testing.assert_array_equal(out[0][0], ho)
+    np.testing.assert_array_equal(out[0][1], co)
+
+
+@pytest.mark.parametrize("precision", ["f32x2", "f32"])
+@pytest.mark.parametrize("res", [9, 11, 33, 61, 121, 305])
+def test_odd_resolutions_blocked_by_default_match_single_steps(sbs, orc, precision, res):
+    """Odd resolutions (rows of 2 r cells, no multiple of four; pole rings of one and several blocks)
+    run blocked by default: the bits of single steps and of the kernel-order oracle, fronts active
+    (first spawn at step 50), volumes."""
+    from soap_bubble_simulation_gb300 import synthetic
+
+    h0 = synthetic.bubble_c0(res, seed=res)
+    h0[res // 3, : res // 2] = 5e-9  # below the 10 nm critical thickness: frozen
+    h0[1, : res // 3] *= 40.0
+    if precision == "f32":
+        h0 = h0.astype(np.float32).astype(np.float64)
+    out = []
+    for single in (False, True):
+        sim = make_sim(sbs, res, precision)
+        if single:
+            set_cpu_blocking(sbs, sim, 1)
+        set64(sbs, sim, h0)
+        sim.step_n(0.01, 47)
+        vols = sim.run_checked(0.01, 34, 17)
+        out.append((field64(sbs, sim), vols))
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_allclose(out[0][1], out[1][1], rtol=1e-12)
+    ref = orc.CpuSim(resolution=res, precision=ORC_PREC[precision])
+    ref.set_field(h0)
+    ref.step_n(0.01, 81)
+    np.testing.assert_array_equal(out[0][0], ref.field())
+
+
+@pytest.mark.parametrize("res", [64, 121, 256])
+def test_pole_rings_of_very_large_words_use_the_wide_sums(sbs, orc, res):
+    """Ring words around the 128-bit sums' range (4096 m) on some or all of the ring's blocks, negative
+    low words, and words below 2^-96 m: the kernel-order oracle's bits."""
+    from soap_bubble_simulation_gb300 import synthetic
+
+    base = synthetic.bubble_c0(res, seed=5)
+    for hi in (4000.0, 5000.0, 1e9):
+        h0 = base.copy()
+        h0[1, 3] = hi
+        h0[res - 2, res : res + 40] = hi / 3.0
+        h0[1, 9] = 1e-30
+        sim = make_sim(sbs, res, "f32x2")
+        set64(sbs, sim, h0)
+        sim.step_n(1e-9, 3)
+        ref = orc.CpuSim(resolution=res, precision=ORC_PREC["f32x2"])
+        ref.set_field(h0)
+        ref.step_n(1e-9, 3)
+        np.testing.assert_array_equal(field64(sbs, sim), ref.field())

@@ -76,3 +76,31 @@ def test_foam_rejects_bad_input(sbs):
     foam = sbs.FoamDrainage([32], [0.01])
     with pytest.raises(ValueError):
         foam.set_thickness(0, np.zeros((32, 32), np.float32))
+
+
+@pytest.mark.parametrize("K,rows", [(1, 8), (2, 16), (4, 32)])
+def test_odd_resolutions_match_single_bubbles(sbs, K, rows):
+    """Odd resolutions (rows of 2 r cells, no multiple of four) beside even ones, with every number
+    of steps per phase: each bubble equal to the single-bubble path."""
+    from soap_bubble_simulation_gb300 import synthetic as S
+
+    res = np.array([3, 33, 61, 64, 75, 121], dtype=np.uint32)
+    rad = np.linspace(0.01, 0.03, res.size).astype(np.float32)
+    foam = sbs.FoamDrainage(res, rad)
+    foam.set_tiles(K, rows)
+    hs = S.foam_fields(res, seed=9)
+    cs = [S.surfactant_noise(int(r), 2 * int(r), seed=int(r)) for r in res]
+    for b in range(res.size):
+        foam.set_thickness(b, hs[b])
+        foam.set_concentration(b, cs[b])
+    foam.run(13)
+    for b, r in enumerate(int(r) for r in res):
+        sim = sbs.GPUDrainageSimulator(None, 500e-9, 2 * r, r)
+        sbs._native.call("sbs_gpu_drainage_set_time_blocking", sim.handle, 1)
+        sim.set_bubble_radius(float(rad[b]))
+        sim.set_thickness_array(hs[b])
+        sim.set_concentration_array(cs[b])
+        sim.run(13)
+        np.testing.assert_array_equal(foam.thickness(b), sim.thickness_array())
+        np.testing.assert_array_equal(foam.concentration(b), sim.concentration_array())
+    foam.close()
