@@ -246,6 +246,12 @@ int allocate(sbs_drainage *h) {
         h->cgeom = wtbc_geometry(h->nt, h->np, k, h->x2);
         if (h->cgeom.nby > 0) h->cpu_k = k;
     }
+    h->rgeom = resident_geometry(h->nt, h->np, h->sem, h->x2);
+    h->resident = h->rgeom.nby > 0;
+    if (h->resident) {
+        SBS_CUDA_TRY(cudaMalloc(&h->halo, resident_halo_bytes(h->rgeom)));
+        SBS_CUDA_TRY(cudaMemset(h->halo, 0, resident_halo_bytes(h->rgeom)));
+    }
     for (int i = 0; i < 2; ++i) {
         SBS_CUDA_TRY(cudaMalloc(&h->part[i], sizeof(FixSum) * 2 * h->geom.nbx));
         SBS_CUDA_TRY(cudaMemset(h->part[i], 0, sizeof(FixSum) * 2 * h->geom.nbx));
@@ -259,6 +265,7 @@ int allocate(sbs_drainage *h) {
             const StepGeom g = wtb_geometry(h->nt, h->np, k);
             vol_blocks = std::max(vol_blocks, (size_t)g.nbx * g.nby);
         }
+    vol_blocks = std::max(vol_blocks, (size_t)h->rgeom.nby);
     size_t slots = 0;
     if (h->sem == SBS_CPU_SEMANTICS)
         for (int k = 2; k <= 4; ++k) {
@@ -314,6 +321,7 @@ void release(sbs_drainage *h) {
     cudaFree(h->sched_dev);
     cudaFree(h->qbuf);
     cudaFree(h->ring_slots);
+    cudaFree(h->halo);
     cudaFree(h->cau_buf);
     if (h->ring_status) cudaFreeHost(h->ring_status);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -328,7 +336,7 @@ bool blocking_selectable(const sbs_drainage *h) { return h->np % 4 == 0; }
 // the final chunk of a run that asked for the map, blocked, with three passes before the final
 // single pass (the map is of the field one pass behind the newest, the buffer the renderer binds).
 bool cau_plan(const sbs_drainage *h, int count, bool last_single) {
-    return h->cau_on && h->sem == SBS_WGSL_SEMANTICS && h->wtb_k > 1 && last_single &&
+    return h->cau_on && h->sem == SBS_WGSL_SEMANTICS && !h->resident && h->wtb_k > 1 && last_single &&
            h->cau_geom.nby > 0 && count - 1 >= kWtbCausticK;
 }
 
@@ -341,6 +349,50 @@ void wait_args(sbs_drainage *h, StepArgs *a) {
     a->wait_cycles = wc.cycles;
     a->extra = (wc.stall & SBS_STALL_GRID_BARRIER) ? 1u : 0u;
     a->inv_np = 1.0 / (double)h->np;
+}
+
+// `count` steps from the current buffer into the other one, as one launch of the resident kernel.
+// WGSL semantics: the current buffer then holds the field one pass behind the newest.
+int enqueue_resident(sbs_drainage *h, int count, float dt, bool vol_last, bool use_sched) {
+    const Consts &k = consts_of(h);
+    const int cur = h->cur;
+    StepArgs a{};
+    a.hin = h->h[cur];
+    a.hout = h->h[cur ^ 1];
+    a.cin = h->c[cur];
+    a.cout = h->c[cur ^ 1];
+    a.lin = h->hl[cur];
+    a.lout = h->hl[cur ^ 1];
+    a.rows = h->rows;
+    a.tfe = use_sched ? h->sched_dev : nullptr;
+    a.vol_w = vol_last ? h->vol_w : nullptr;
+    a.vol_partials = h->vol_partials;
+    a.vol_counter = h->vol_counter;
+    a.vol_out = h->vol_out;
+    a.vol_index = h->vol_index;
+    a.nt = h->nt;
+    a.np = h->np;
+    a.pitch = (int)h->pitch;
+    a.rb = h->rgeom.rb;
+    a.marangoni = h->sem == SBS_WGSL_SEMANTICS && h->params.marangoni_enabled ? 1 : 0;
+    a.crit = k.crit;
+    a.b = k.b;
+    a.DR2 = k.DR2;
+    a.DsR2 = k.DsR2;
+    a.Gt = k.Gt;
+    a.M = k.M;
+    a.dt = dt;
+    wait_args(h, &a);
+    ResidentArgs ra{};
+    ra.halo = h->halo;
+    ra.hprev = h->h[cur];
+    ra.cprev = h->c[cur];
+    ra.tag0 = h->halo_tag;
+    ra.stall = a.extra ? 1u << 30 : 0u;
+    ra.steps = count;
+    h->halo_tag += (unsigned)count + 1u;
+    SBS_CUDA_TRY(launch_resident(h->sem, h->x2, a, ra, h->rgeom, h->stream));
+    return SBS_OK;
 }
 
 // Enqueues `count` steps starting from buffer `start`; returns the buffer holding the result.
@@ -517,7 +569,11 @@ int run_chunk(sbs_drainage *h, int count, double dt, bool vol_last, bool last_si
         for (int i = 0; i < count; ++i) h->current_time += (double)h->params.dt;
     }
     int end = h->cur;
-    if (count < kGraphMin) {
+    if (h->resident) {
+        int rc = enqueue_resident(h, count, dtf, vol_last, use_sched);
+        if (rc) return rc;
+        end = h->cur ^ 1;
+    } else if (count < kGraphMin) {
         int rc = enqueue_steps(h, h->cur, count, dtf, vol_last, use_sched, last_single, &end);
         if (rc) return rc;
     } else {
@@ -561,14 +617,15 @@ int run_chunk(sbs_drainage *h, int count, double dt, bool vol_last, bool last_si
     return SBS_OK;
 }
 
-// After the stream has drained: a timed-out ring exchange of the blocked CPU-semantics step turns
-// into SBS_E_TIMEOUT, and its slots (whose tags count on) and the status are cleared for the next call.
+// After the stream has drained: a timed-out ring exchange of the blocked CPU-semantics step, or row
+// exchange of the resident kernel, turns into SBS_E_TIMEOUT, and the ring's slots (whose tags count
+// on) and the status are cleared for the next call. The row exchange's step numbers never repeat.
 int check_ring_status(sbs_drainage *h) {
     if (!h->ring_status || *(volatile unsigned *)h->ring_status == 0u) return SBS_OK;
     *(volatile unsigned *)h->ring_status = 0u;
     SBS_CUDA_TRY(cudaMemsetAsync(h->ring_slots, 0, h->ring_bytes, h->stream));
     SBS_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    return set_error(SBS_E_TIMEOUT, "drainage: a wait for another block's ring sum timed out");
+    return set_error(SBS_E_TIMEOUT, "drainage: a wait for another block's row or ring sum timed out");
 }
 
 // Advances n steps in chunks; a volume check follows every check_every-th step (0 = none).
@@ -698,6 +755,7 @@ int create_common(sbs_drainage *h) {
 
 namespace sbs {
 int drainage_run_async(sbs_drainage *h, uint32_t passes) { return run_steps(h, 0.0, passes, 0); }
+int drainage_check(sbs_drainage *h) { return check_ring_status(h); }
 }  // namespace sbs
 
 extern "C" {
@@ -1204,6 +1262,7 @@ int sbs_gpu_drainage_set_time_blocking(sbs_drainage *h, int steps_per_launch) {
     if (steps_per_launch > 1 && !(blocking_selectable(h) && wtb_supported(h->nt, h->np)))
         return set_error(SBS_E_INVALID, "time blocking needs grid_width a multiple of 4 (got %d)", h->np);
     destroy_graphs(h);
+    h->resident = false;
     h->wtb_k = steps_per_launch > 1 ? steps_per_launch : 0;
     if (h->wtb_k) h->wgeom = wtb_geometry(h->nt, h->np, h->wtb_k);
     return SBS_OK;
@@ -1231,6 +1290,7 @@ int sbs_drainage_set_time_blocking(sbs_drainage *h, int steps_per_launch) {
     }
     SBS_CUDA_TRY(cudaStreamSynchronize(h->stream));
     destroy_graphs(h);
+    h->resident = false;
     h->cpu_k = steps_per_launch > 1 ? steps_per_launch : 0;
     h->cgeom = g;
     return SBS_OK;

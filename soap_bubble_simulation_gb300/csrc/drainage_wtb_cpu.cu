@@ -34,9 +34,9 @@
 // stencil's ring values, then the fronts thin their cells.
 //
 // The per-cell arithmetic is cpu_row() (cell.cuh), which gives the bits of the single-step kernel, and
-// the front factor the double-float
-// product of the single-step kernel, so K single steps and one launch of this give the same bits
-// (the ring sums are exact, which makes them independent of the summation order).
+// the front factor the double-float product of the single-step kernel, so K single steps and one
+// launch of this give the same bits (the ring sums are exact, which makes them independent of the
+// summation order).
 #include <cuda_runtime.h>
 
 #include "cell.cuh"

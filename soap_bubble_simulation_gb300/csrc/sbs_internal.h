@@ -55,8 +55,10 @@ WaitConfig wait_config();
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t s);
 
 // WGSL-semantics passes (params.dt each) enqueued on the handle's stream without a final
-// synchronisation (sbs_gpu_drainage_run minus the wait).
+// synchronisation (sbs_gpu_drainage_run minus the wait). After the caller has synchronised the
+// stream, drainage_check reports a wait of those passes that ran out.
 int drainage_run_async(sbs_drainage *h, uint32_t passes);
+int drainage_check(sbs_drainage *h);
 
 // Area-weighted (sin theta) mean of each bubble's current thickness field of a batched foam, in
 // nm, into out[cap] (device memory); *nb = the batch's bubble count (out is written only when
@@ -137,6 +139,21 @@ constexpr int kWtbCausticK = 3;
 StepGeom wtbc_geometry(int nt, int np, int K, int x2);
 size_t wtbc_ring_bytes(const StepGeom &g);
 cudaError_t launch_wtbc(int K, int x2, const StepArgs &a, const StepGeom &g, cudaStream_t s);
+// A chunk of steps in one launch, the field held on the chip (drainage_resident.cu): nby blocks of
+// wx warps, at most rb rows each, all resident at once. nby == 0: the grid is not supported. The
+// blocks exchange rows through resident_halo_bytes(g) of words that carry the number of their step;
+// no number may come up twice while the words last, so tag0 grows by steps + 1 with every launch.
+struct ResidentArgs {
+    unsigned long long *halo;
+    float *hprev, *cprev;  // WGSL semantics: where the field one pass behind the newest goes
+    unsigned tag0;
+    unsigned stall;        // added to the number a reader waits for (nonzero only in the timeout test)
+    int steps;
+};
+StepGeom resident_geometry(int nt, int np, int semantics, int x2);
+size_t resident_halo_bytes(const StepGeom &g);
+cudaError_t launch_resident(int semantics, int x2, const StepArgs &a, const ResidentArgs &ra, const StepGeom &g,
+                            cudaStream_t s);
 // x2: compensated f32x2 thickness (hi + lo words); CPU semantics only.
 cudaError_t launch_step(int semantics, int x2, const StepArgs &a, const StepGeom &g, cudaStream_t s);
 // Writes the pole rows of `h` (and `hl`, if not null) from the ring partials of the last step.
@@ -242,6 +259,10 @@ struct sbs_drainage {
     sbs::StepGeom wgeom{};
     int cpu_k = 0;  // steps per temporally blocked launch (CPU semantics; 0 = single steps only)
     sbs::StepGeom cgeom{};
+    bool resident = false;                     // chunks run through the resident kernel
+    sbs::StepGeom rgeom{};
+    unsigned long long *halo = nullptr;        // its row exchange
+    unsigned halo_tag = 0;                     // the last step number used there
     unsigned long long *ring_slots = nullptr;  // the blocked step's ring exchange (CPU semantics), then the
     size_t ring_bytes = 0;                     // waits' status word in the last 8 of ring_bytes
     unsigned *ring_status = nullptr;   // host-mapped timeout word

@@ -903,6 +903,7 @@ int sbs_surrogate_rollout(sbs_surrogate *s, sbs_drainage *d, uint32_t passes, ui
         st.rollouts++;
     }
     SBS_CUDA_TRY(cudaStreamSynchronize(d->stream));
+    if ((rc = drainage_check(d))) return rc;
     if ((rc = tc_status(s))) return rc;
     if (stats) *stats = st;
     return SBS_OK;

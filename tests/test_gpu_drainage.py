@@ -599,3 +599,59 @@ def test_pole_rings_of_very_large_words_use_the_wide_sums(sbs, orc, res):
         ref.set_field(h0)
         ref.step_n(1e-9, 3)
         np.testing.assert_array_equal(field64(sbs, sim), ref.field())
+
+
+@pytest.mark.parametrize("marangoni", [0, 1])
+@pytest.mark.parametrize("W,H", [(3, 3), (7, 4), (128, 3), (130, 90), (255, 160), (640, 310), (1027, 500), (2048, 160)])
+def test_resident_chunks_match_single_steps(sbs, orc, W, H, marangoni):
+    """Grids that stay on the chip for a chunk of passes (default): one and several rows per block,
+    one to sixteen warps per row, the seam inside a lane's window, chunks of 256 and a remainder, the
+    field one pass behind the newest, volumes: the bits of single steps."""
+    from soap_bubble_simulation_gb300 import synthetic
+
+    h = synthetic.smooth_modes(H, W, seed=W + H).astype(np.float32)
+    h[H // 2, : W // 3] = 25e-9  # below the critical thickness
+    c = synthetic.surfactant_noise(H, W, seed=H)
+    c[H // 2, -1] = 1.0
+    out = []
+    for single in (False, True):
+        sim = sbs.GPUDrainageSimulator(None, 500e-9, W, H)
+        if single:
+            set_blocking(sbs, sim, 1)
+        sim.set_thickness_array(h)
+        sim.set_concentration_array(c)
+        sim.set_marangoni_enabled(bool(marangoni))
+        sim.run(1)
+        sim.run(2)
+        vols = sim.run_checked(0.001, 300, 130)
+        stale = sim.current_buffer()
+        v = sbs.film_volume_device(stale.ptr, H, W, stale.pitch, 0.025)
+        out.append((sim.thickness_array(), sim.concentration_array(), vols, v, sim.current_time()))
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+    np.testing.assert_allclose(out[0][2], out[1][2], rtol=1e-12)
+    assert out[0][3] == pytest.approx(out[1][3], rel=1e-12) and out[0][4] == out[1][4]
+
+
+@pytest.mark.parametrize("precision", ["f32x2", "f32"])
+@pytest.mark.parametrize("res", [3, 4, 64, 153, 200, 320, 330])
+def test_resident_cpu_chunks_match_single_steps(sbs, precision, res):
+    """The same in DrainageSimulator semantics, with fronts (the first at step 50) over several rows of
+    a block, and both poles in one block at the smallest sizes."""
+    from soap_bubble_simulation_gb300 import synthetic
+
+    h0 = synthetic.bubble_c0(res, seed=res)
+    h0[res // 3, : res // 2] = 5e-9
+    out = []
+    for single in (False, True):
+        sim = make_sim(sbs, res, precision)
+        if single:
+            set_cpu_blocking(sbs, sim, 1)
+        set64(sbs, sim, h0)
+        sim.step(0.01)
+        sim.step_n(0.01, 300)
+        vols = sim.run_checked(0.01, 40, 20)
+        out.append((field64(sbs, sim), vols, sim.active_tfe_count()))
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_allclose(out[0][1], out[1][1], rtol=1e-12)
+    assert out[0][2] == out[1][2] >= 1

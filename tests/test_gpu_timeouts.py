@@ -164,3 +164,31 @@ def test_training_convolution_waits_time_out_then_recover(sbs, short_waits):
     losses = s.train(4, 60, batch=2, lr=3e-3, seed=1)
     assert np.isfinite(losses).all() and losses[-10:].mean() < losses[:3].mean()
     s.close()
+
+
+def test_resident_row_exchange_times_out_then_recovers(sbs, short_waits):
+    """Small grids advance in one launch whose blocks wait for their neighbours' rows; with those
+    waits unsatisfiable a GPUDrainageSimulator run reports the timeout, and afterwards the handle
+    steps like a fresh one (the DrainageSimulator's are covered above: 64 x 128 is such a grid)."""
+    from soap_bubble_simulation_gb300 import synthetic
+
+    N = short_waits
+    h0 = synthetic.smooth_modes(40, 90, seed=2).astype(np.float32)
+    c0 = synthetic.surfactant_noise(40, 90, seed=3)
+    sims = [sbs.GPUDrainageSimulator(None, 500e-9, 90, 40) for _ in range(2)]
+
+    def load(sim):
+        sim.set_thickness_array(h0)
+        sim.set_concentration_array(c0)
+
+    load(sims[0])
+    N.call("sbs_set_stall_injection", N.STALL_GRID_BARRIER)
+    with pytest.raises(sbs.SbsError) as e:
+        sims[0].run(5)
+    assert e.value.code == N.SBS_E_TIMEOUT
+    N.call("sbs_set_stall_injection", 0)
+    for s in sims:
+        load(s)
+        s.run(20)
+    np.testing.assert_array_equal(sims[0].thickness_array(), sims[1].thickness_array())
+    np.testing.assert_array_equal(sims[0].concentration_array(), sims[1].concentration_array())
