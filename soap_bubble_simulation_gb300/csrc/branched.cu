@@ -197,7 +197,9 @@ __device__ __forceinline__ float sample_uv(const TraceArgs &a, float u, float v)
     return __ldg(a.thickness + (size_t)y * a.pitch + x);
 }
 
-__device__ __forceinline__ void deposit(const TraceArgs &a, float u, float v, float intensity) {
+// The bilinear deposit; with several lanes to a ray, the first adds the upper row and the second the lower.
+template <int L>
+__device__ __forceinline__ void deposit(const TraceArgs &a, float u, float v, float intensity, int sub) {
     const uint32_t tw = a.p.tex_width, th = a.p.tex_height;
     const float fx = fminf(fmaxf(u, 0.0f), 1.0f) * (float)(tw - 1u);
     const float fy = fminf(fmaxf(v, 0.0f), 1.0f) * (float)(th - 1u);
@@ -206,13 +208,22 @@ __device__ __forceinline__ void deposit(const TraceArgs &a, float u, float v, fl
     const float sx = fx - floorf(fx), sy = fy - floorf(fy);
     const float w00 = (1.0f - sx) * (1.0f - sy), w10 = sx * (1.0f - sy), w01 = (1.0f - sx) * sy, w11 = sx * sy;
     const float base = intensity * 256.0f;
-    atomicAdd(a.tex + y0 * tw + x0, (uint32_t)(base * w00));
-    atomicAdd(a.tex + y0 * tw + x1, (uint32_t)(base * w10));
-    atomicAdd(a.tex + y1 * tw + x0, (uint32_t)(base * w01));
-    atomicAdd(a.tex + y1 * tw + x1, (uint32_t)(base * w11));
+    if (L == 1 || sub == 0) {
+        atomicAdd(a.tex + y0 * tw + x0, (uint32_t)(base * w00));
+        atomicAdd(a.tex + y0 * tw + x1, (uint32_t)(base * w10));
+    }
+    if (L == 1 || sub == 1) {
+        atomicAdd(a.tex + y1 * tw + x0, (uint32_t)(base * w01));
+        atomicAdd(a.tex + y1 * tw + x1, (uint32_t)(base * w11));
+    }
 }
 
-__global__ void __launch_bounds__(128) trace_kernel(TraceArgs a) {
+// L lanes trace a ray together (1, 2 or 4): all hold its state and do the same operations, but form
+// different scatterers' terms (two each per round), which every lane then adds in list order through
+// shuffles. A ray's step is one chain of ~1,700 instructions, so few rays leave the chip waiting (ncu
+// at 32,768 rays: issue 30 % used, warps waiting for their own results).
+template <int L>
+__global__ void __launch_bounds__(128) trace_kernel(const TraceArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
     sbs_scatterer *sc = reinterpret_cast<sbs_scatterer *>(smem);
     float *scut = reinterpret_cast<float *>(sc + a.nscat);  // each scatterer's cutoff 4.5 / inv_sigma_sq
@@ -225,9 +236,10 @@ __global__ void __launch_bounds__(128) trace_kernel(TraceArgs a) {
     for (int k = threadIdx.x; k <= kGrid * kGrid; k += blockDim.x) off[k] = a.list_off[k];
     for (int k = threadIdx.x; k < a.nlist; k += blockDim.x) lst[k] = a.list[k];
     __syncthreads();
-    const uint32_t ray = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t ray = (blockIdx.x * blockDim.x + threadIdx.x) / L;
+    const int lane = threadIdx.x & 31, sub = lane % L, lane0 = lane - sub;
     const sbs_branched_params &p = a.p;
-    if (ray >= p.num_rays) return;
+    bool alive = ray < p.num_rays;  // the warp stays together until its last ray ends
     const Setup &s = a.s;
     const float rand1 = hash21((float)ray * 0.1f, 0.0f);
     const float rand2 = hash21((float)ray * 0.1f + 100.0f, 1.0f);
@@ -245,6 +257,7 @@ __global__ void __launch_bounds__(128) trace_kernel(TraceArgs a) {
     const float max_v = fminf(p.patch_center_v + p.patch_half_size, 1.0f);
     const float gw = 1.0f - p.particle_weight;
     for (uint32_t step = 0; step < p.ray_steps; ++step) {
+        if (!__any_sync(0xffffffffu, alive)) break;
         // pos_3d = normalize(entry + tangent1 * pos.x + tangent2 * pos.y); uv = normal_to_uv(pos_3d)
         const float qx = s.ex + s.t1x * posx + s.t2x * posy;
         const float qy = s.ey + s.t1y * posx + s.t2y * posy;
@@ -264,15 +277,16 @@ __global__ void __launch_bounds__(128) trace_kernel(TraceArgs a) {
         // numerators of 0 or at least 1e-7: sums and products with pi's own rounding
         const float u = quotient(atan2_as(nz, nx) + kPi, 2.0f * kPi, 1.0f / (2.0f * kPi));
         const float v = quotient(acos_as(fminf(fmaxf(ny, -1.0f), 1.0f)), kPi, 1.0f / kPi);
-        if (patch) {
+        if (!alive) {
+        } else if (patch) {
             const float du = fabsf(u - p.patch_center_u), dv = fabsf(v - p.patch_center_v);
             if (du <= p.patch_half_size && dv <= p.patch_half_size) {
                 const float lu = fminf(fmaxf((u - min_u) / fmaxf(max_u - min_u, 0.001f), 0.0f), 1.0f);
                 const float lv = fminf(fmaxf((v - min_v) / fmaxf(max_v - min_v, 0.001f), 0.0f), 1.0f);
-                deposit(a, lu, lv, intensity * 0.15f);
+                deposit<L>(a, lu, lv, intensity * 0.15f, sub);
             }
         } else {
-            deposit(a, u, v, intensity * 0.15f);
+            deposit<L>(a, u, v, intensity * 0.15f, sub);
         }
         // GRIN kick: thickness_gradient_uv (:197-211)
         const float eps = 0.01f;
@@ -290,29 +304,35 @@ __global__ void __launch_bounds__(128) trace_kernel(TraceArgs a) {
 #pragma unroll
             for (int w = 0; w < 4; ++w, base += 32u) {
                 uint32_t m = w == 0 ? words.x : w == 1 ? words.y : w == 2 ? words.z : words.w;
-                while (m) {  // two scatterers at a time, their terms added in order
-                    const uint32_t i0 = lst[base + (uint32_t)__ffs((int)m) - 1u];
-                    m &= m - 1u;
-                    const bool two = m != 0u;
-                    const uint32_t i1 = two ? lst[base + (uint32_t)__ffs((int)m) - 1u] : i0;
-                    m &= m - 1u;
-                    const sbs_scatterer q0 = sc[i0], q1 = sc[i1];
-                    const float dx0 = u - q0.pos_u, dy0 = v - q0.pos_v, dx1 = u - q1.pos_u, dy1 = v - q1.pos_v;
-                    const float r0 = dx0 * dx0 + dy0 * dy0, r1 = dx1 * dx1 + dy1 * dy1;
-                    const bool in0 = !(r0 > scut[i0]), in1 = two && !(r1 > scut[i1]);  // else it adds zero
-                    if (!(in0 || in1)) continue;
-                    const float x0 = -r0 * q0.inv_sigma_sq, x1 = -r1 * q1.inv_sigma_sq;
-                    float e0 = exp_cw_near(x0), e1 = exp_cw_near(x1);
-                    if (!(fabsf(x0) < 80.0f)) e0 = exp_cw(x0);
-                    if (!(fabsf(x1) < 80.0f)) e1 = exp_cw(x1);
-                    const float cx0 = dx0 * q0.strength * q0.inv_sigma_sq * 2.0f * e0;
-                    const float cy0 = dy0 * q0.strength * q0.inv_sigma_sq * 2.0f * e0;
-                    const float cx1 = dx1 * q1.strength * q1.inv_sigma_sq * 2.0f * e1;
-                    const float cy1 = dy1 * q1.strength * q1.inv_sigma_sq * 2.0f * e1;
-                    fx = in0 ? fx + cx0 : fx;
-                    fy = in0 ? fy + cy0 : fy;
-                    fx = in1 ? fx + cx1 : fx;
-                    fy = in1 ? fy + cy1 : fy;
+                while (L == 1 ? m != 0u : __any_sync(0xffffffffu, m != 0u)) {  // 2 L scatterers a round
+                    float cx[2], cy[2];
+#pragma unroll
+                    for (int j = 0; j < 2 * L - 2; ++j)  // to this lane's two
+                        if (j < 2 * sub) m &= m - 1u;
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const bool some = m != 0u;
+                        const uint32_t idx = some ? lst[base + (uint32_t)__ffs((int)m) - 1u] : 0u;
+                        m &= m - 1u;
+                        const sbs_scatterer q = sc[idx];
+                        const float dx = u - q.pos_u, dy = v - q.pos_v;
+                        const float r2 = dx * dx + dy * dy;
+                        const bool in = some && !(r2 > scut[idx]);
+                        const float x = -r2 * q.inv_sigma_sq;
+                        float e = exp_cw_near(x);
+                        if (in && !(fabsf(x) < 80.0f)) e = exp_cw(x);
+                        // beyond its cutoff a scatterer adds nothing: a zero changes no sum here
+                        cx[j] = in ? dx * q.strength * q.inv_sigma_sq * 2.0f * e : 0.0f;
+                        cy[j] = in ? dy * q.strength * q.inv_sigma_sq * 2.0f * e : 0.0f;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 2 * L - 2; ++j)  // and past the others'
+                        if (j >= 2 * sub) m &= m - 1u;
+#pragma unroll
+                    for (int j = 0; j < 2 * L; ++j) {
+                        fx += L == 1 ? cx[j] : __shfl_sync(0xffffffffu, cx[j % 2], lane0 + j / 2);
+                        fy += L == 1 ? cy[j] : __shfl_sync(0xffffffffu, cy[j % 2], lane0 + j / 2);
+                    }
                 }
             }
         }
@@ -334,9 +354,14 @@ __global__ void __launch_bounds__(128) trace_kernel(TraceArgs a) {
         posy = posy + vy * dt;
         intensity = intensity * (1.0f - p.intensity_falloff);
         // |pos| > 2.5: the square root rounds to more than 2.5 from the second float above 6.25 on
-        if (posx * posx + posy * posy > 6.2500005f || intensity < 0.01f) break;
+        if (posx * posx + posy * posy > 6.2500005f || intensity < 0.01f) alive = false;
     }
 }
+
+// More lanes to a ray while the chip has no other work to overlap. 400 steps, ms with 1, 2 and 4 lanes:
+// 2,000 rays 2.00, 1.50, 1.33; 8,192 1.99, 1.49, 1.41; 16,384 1.99, 1.63, 1.80; 32,768 2.26, 2.28,
+// 2.66; 60,000 3.39, 3.72, 4.26. (All 800 scatterers' neighbourhood lists, one lane: 5.08 at 32,768.)
+int lanes_per_ray(uint32_t rays) { return rays <= 10000u ? 4 : rays <= 24000u ? 2 : 1; }
 
 __global__ void fade_kernel(uint32_t *tex, size_t n) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -580,10 +605,14 @@ int sbs_branched_flow(const sbs_branched_params *p, const float *thickness, uint
         a.tex = d_tex;
         cull_kernel<<<(unsigned)((4 * mask_n + 127) / 128), 128, 0, s>>>(a, reinterpret_cast<uint32_t *>(d_mask));
         const size_t smem = sc_b + sizeof(float) * nscat + off_b + sizeof(uint16_t) * lst.size() + 16;
-        e = cudaFuncSetAttribute(trace_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const int lanes = lanes_per_ray(p->num_rays);
+        const void *fn = lanes == 1 ? (const void *)trace_kernel<1>
+                         : lanes == 2 ? (const void *)trace_kernel<2> : (const void *)trace_kernel<4>;
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess) {
-            trace_kernel<<<(p->num_rays + 127) / 128, 128, smem, s>>>(a);
-            e = cudaGetLastError();
+            void *args[] = {(void *)&a};
+            const unsigned per_block = 128u / (unsigned)lanes;
+            e = cudaLaunchKernel(fn, dim3((p->num_rays + per_block - 1) / per_block), dim3(128), args, smem, s);
         }
     }
     if (e == cudaSuccess && mem == SBS_MEM_HOST) e = cudaMemcpyAsync(texture, d_tex, 4 * tex_n, cudaMemcpyDeviceToHost, s);

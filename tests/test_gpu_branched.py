@@ -61,3 +61,20 @@ def test_bad_arguments(sbs, br):
     with pytest.raises(sbs.SbsError):
         br.branched_flow_step(p, field(), br.generate_scatterers(br.BranchedFlowParams.default()),
                               np.zeros((256, 1), np.uint32))
+
+
+@pytest.mark.parametrize("rays", [1, 33, 10000, 10001, 24000, 24001])
+def test_every_number_of_lanes_per_ray_matches_oracle(sbs, orc, br, rays):
+    """Ray counts at the edges of the rule that gives a ray 4, 2 or 1 lanes; scatterers of very
+    different cutoffs (one covers the whole film, one nothing), more than 128 of them in a cell's list."""
+    p = br.BranchedFlowParams.default()
+    p.num_rays, p.patch_enabled, p.ray_steps, p.num_scatterers = rays, 0, 60, 700
+    g = np.random.default_rng(rays)
+    sc = br.generate_scatterers(p, time=0.5)
+    sc[:200, :2] = 0.45 + 0.1 * g.random((200, 2))
+    sc[5, 3], sc[6, 3], sc[7, 3] = 0.5, 1e9, 40.0
+    th = field(scale=2e4)
+    tex0 = np.zeros((p.tex_height, p.tex_width), np.uint32)
+    got = br.branched_flow_step(p, th, sc, tex0, fade=False)
+    assert np.array_equal(got, orc.branched_flow(p, th, sc, tex0, False))
+    assert got.sum() > 0
