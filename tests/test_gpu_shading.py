@@ -93,6 +93,29 @@ def test_fragments_with_branched_flow(sbs, orc, sh):
         assert (got[:, 0] > plain[:, 0] + 1e-3).mean() > (0.01 if patch else 0.3)
 
 
+@pytest.mark.parametrize("film_time", [-70.0, 1e6, -3e6, 2.6e7, 1.1e8, -4e8, 1e12])
+def test_noise_beyond_the_tables_matches_oracle(sbs, orc, sh, film_time):
+    """Lattice coordinates below zero, about 2^23 and far beyond (the tabulated noise ends at 2^23)."""
+    lut = sh.default_lut(1.33)
+    nn, wp = sphere_fragments(5000, 9)
+    u = sh.BubbleUniform.default()
+    u.film_time = film_time
+    got = sh.shade_fragments(u, (0.0, 0.06, 0.19), lut, nn, wp)
+    want = orc.shade_fragments(u, (0.0, 0.06, 0.19), lut, nn, wp)
+    assert np.abs(got - want).max() <= 2e-5
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, 400001])
+def test_fragment_counts_match_oracle(sbs, orc, sh, n):
+    """One thread, a block's edges, and more fragments than the device has threads (blocks take turns)."""
+    lut = sh.default_lut(1.33)
+    nn, wp = sphere_fragments(n, 11)
+    u = sh.BubbleUniform.default()
+    got = sh.shade_fragments(u, (0.0, 0.06, 0.19), lut, nn, wp)
+    want = orc.shade_fragments(u, (0.0, 0.06, 0.19), lut, nn, wp)
+    assert np.abs(got - want).max() <= 2e-5
+
+
 @pytest.mark.parametrize("w,h,yaw,pitch", [(160, 90, 0.0, 0.3), (97, 131, 1.1, -0.4), (64, 64, 2.5, 1.2)])
 def test_frame_matches_oracle(sbs, orc, sh, w, h, yaw, pitch):
     lut = sh.default_lut(1.33)
@@ -112,6 +135,19 @@ def test_frame_matches_oracle(sbs, orc, sh, w, h, yaw, pitch):
     hit = np.any(np.abs(lin[..., :3] - bg) > 1e-6, axis=-1)
     r = math.tan(math.asin(0.025 / 0.2)) / math.tan(math.radians(22.5))
     assert abs(hit.mean() - math.pi * r * r / (4 * w / h)) < 0.02
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (17, 16), (1021, 607)])
+def test_frame_sizes_match_oracle(sbs, orc, sh, w, h):
+    """One pixel, a tile's edge, and more tiles than the device takes at once (blocks take turns)."""
+    lut = sh.default_lut(1.33)
+    cam = sh.Camera(aspect=w / h)
+    u = sh.BubbleUniform.default()
+    lin = sh.render_frame(u, cam, w, h, lut=lut, linear=True)
+    rgba8 = sh.render_frame(u, cam, w, h, lut=lut)
+    want8, want_lin = orc.shade_frame(u, cam.view_proj(), cam.position(), sh.HEADLESS_RADIUS, lut, w, h)
+    assert (np.abs(lin - want_lin).max(axis=-1) <= 1e-4).mean() >= 0.97
+    assert (np.abs(rgba8.astype(int) - want8.astype(int)).max(axis=-1) <= 1).mean() >= 0.99
 
 
 def test_device_memory_frame(sbs, sh):
