@@ -28,6 +28,7 @@
 #include <cstring>
 #include <vector>
 
+#include "exact.cuh"
 #include "sbs_internal.h"
 
 namespace sbs {
@@ -111,13 +112,6 @@ __device__ __forceinline__ float exp_cw_near(float x) {
     return __int_as_float(__float_as_int(p) + ((__float_as_int(t) - 0x4b400000) << 23));
 }
 
-// a / b rounded once, from r = 1 / b rounded: q = a r, then q + (a - q b) r (Markstein, IBM J. Res.
-// Dev. 34, 1990). The residual is exact while |a| is not tiny (kTiny); a = 0 is fine too.
-constexpr float kTiny = 0x1p-90f;
-__device__ __forceinline__ float quotient(float a, float b, float r) {
-    const float q = a * r;
-    return fmaf(fmaf(-q, b, a), r, q);
-}
 __device__ __forceinline__ float divide(float a, float b, float r) {  // any a
     return fabsf(a) < kTiny ? a / b : quotient(a, b, r);
 }

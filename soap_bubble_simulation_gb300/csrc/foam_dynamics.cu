@@ -8,8 +8,8 @@
 // 3 (r_a + r_b) contributes exact zeros (no van der Waals, repulsion or adhesion term applies),
 // and adding a zero leaves a sum unchanged. So a walk over a neighbour list sorted by bubble
 // index, holding every pair that can come within that range, forms the reference's f32 sums
-// exactly, in O(n) instead of O(n^2): one thread per bubble, or for small foams a few lanes that
-// evaluate consecutive entries together and add them in order.
+// exactly, in O(n) instead of O(n^2): a few lanes per bubble evaluate consecutive entries together and
+// add them in order.
 //
 // Neighbour list (Verlet list): bubble k lists every j with |p_j - p_k| < 3 (r_k + r_j) + skin at
 // the time of the build; it stays complete while no bubble has moved skin / 2 since (two bubbles
@@ -40,6 +40,7 @@
 #include <cstring>
 #include <vector>
 
+#include "exact.cuh"
 #include "sbs_internal.h"
 
 namespace sbs {
@@ -60,7 +61,7 @@ enum Fault : uint32_t { kFaultNone = 0, kFaultCapacity = 1, kFaultDense = 2, kFa
 struct Ctl {
     uint32_t n[2];          // bubble count; a merge pass reads n[p] and writes n[p ^ 1]
     uint32_t next_id;       // BubbleCluster::next_id
-    uint32_t need_rebuild;  // set by the connection pass (displacement) and by a merge
+    uint32_t stale;         // the step after which the list needs a rebuild (displacement, a merge), kNone if it holds
     uint32_t go;            // the rebuild enqueued for this step runs
     uint32_t fault;         // Fault
     uint32_t steps_done;    // steps whose force pass ran in the current call
@@ -83,10 +84,9 @@ struct Bufs {
 
 __device__ __forceinline__ float len3(float x, float y, float z) { return sqrtf(x * x + y * y + z * z); }
 
-// x^1.5 for x > 0: p = x s with s the correctly rounded sqrt(x), plus the exact FMA residuals of the
+// x^1.5 for x > 0 and s the correctly rounded sqrt(x): p = x s, plus the exact FMA residuals of the
 // product (x s - p) and of the root (x - s^2, scaled by x / (2 sqrt x) ~ s / 2).
-__host__ __device__ __forceinline__ float pow15(float x) {
-    const float s = sqrtf(x);
+__host__ __device__ __forceinline__ float pow15(float x, float s) {
     const float p = x * s;
     const float e = fmaf(x, s, -p);
     const float r = fmaf(-s, s, x);
@@ -117,7 +117,7 @@ __device__ __forceinline__ void pair_force(const Phys &P, float4 a, float4 b, fl
     }
     const float overlap = sum_radii - distance;
     if (overlap > 0.0f) {
-        const float rep = P.stiffness * pow15(overlap);
+        const float rep = P.stiffness * pow15(overlap, sqrtf(overlap));
         fx = fx - ux * rep;
         fy = fy - uy * rep;
         fz = fz - uz * rep;
@@ -129,6 +129,48 @@ __device__ __forceinline__ void pair_force(const Phys &P, float4 a, float4 b, fl
         fx = fx + ux * adh;
         fy = fy + uy * adh;
         fz = fz + uz * adh;
+    }
+}
+
+// The force of pair_force on `me` (negated where the other one is the lower index), the same bits without
+// its divisions and branches: one reciprocal of the distance serves the direction and, squared and
+// corrected, the attraction. What lies outside the ranges where the residuals are
+// exact (components or a strength below 2^-90, radii of 2^60) is left to pair_force.
+__device__ __forceinline__ void pair_force_near(const Phys &P, const float4 &me, const float4 &o, bool lower, float &fx,
+                                                float &fy, float &fz) {
+    const float dx = o.x - me.x, dy = o.y - me.y, dz = o.z - me.z;
+    const float d2 = dx * dx + dy * dy + dz * dz;
+    const float sum_radii = me.w + o.w;
+    float r;
+    const float distance = sqrt_near(d2, r);
+    r = recip_near(distance, r);
+    const float dd = distance * distance;
+    const float rr = recip_near(dd, r * r);
+    const float strength = P.vdw * (lower ? o.w : me.w) * (lower ? me.w : o.w);
+    const bool in = distance >= 1e-6f && distance < sum_radii * 3.0f;
+    float s = distance > sum_radii ? quotient(strength, dd, rr) : 0.0f;
+    const float overlap = sum_radii - distance;
+    if (in && overlap > 0.0f) {  // at least 2^-43, an ulp of either
+        float rs;
+        const float root = sqrt_near(overlap, rs);
+        s = -(P.stiffness * pow15(overlap, root));
+    }
+    const float ct = sum_radii * 1.2f;
+    const float adh = distance < ct && distance > sum_radii * 0.95f ? 2.0f * (ct - distance) : 0.0f;
+    const float ux = quotient(dx, distance, r), uy = quotient(dy, distance, r), uz = quotient(dz, distance, r);
+    fx = in ? ux * s + ux * adh : 0.0f;
+    fy = in ? uy * s + uy * adh : 0.0f;
+    fz = in ? uz * s + uz * adh : 0.0f;
+    // twice the bits less one: the sign is gone and a zero is the largest
+    const auto mag = [](float x) { return 2u * __float_as_uint(x) - 1u; };
+    const unsigned least = min(min(mag(dx), mag(dy)), min(mag(dz), mag(strength)));
+    if (!(sum_radii < 0x1p60f) || (in && (least < mag(kTiny) || !(fabsf(strength) < 0x1p60f)))) {
+        pair_force(P, lower ? o : me, lower ? me : o, fx, fy, fz);
+        if (lower) {
+            fx = -fx;
+            fy = -fy;
+            fz = -fz;
+        }
     }
 }
 
@@ -185,7 +227,7 @@ __global__ void __launch_bounds__(1024) list_begin_kernel(ListArgs a, int forced
     __shared__ float s_max[32];
     __shared__ int s_go;
     Ctl *c = a.ctl;
-    if (threadIdx.x == 0) s_go = (c->fault == kFaultNone) && (forced || c->need_rebuild);
+    if (threadIdx.x == 0) s_go = (c->fault == kFaultNone) && (forced || c->stale != kNone);
     __syncthreads();
     if (!s_go) {
         if (threadIdx.x == 0) c->go = 0;
@@ -208,7 +250,7 @@ __global__ void __launch_bounds__(1024) list_begin_kernel(ListArgs a, int forced
             c->cell = cell;
             c->rmax = m;
             c->skin = skin;
-            c->need_rebuild = 0;
+            c->stale = kNone;
             c->go = 1;
         }
     }
@@ -598,35 +640,49 @@ struct DynArgs {
     const uint32_t *perm;  // thread t of the force and connection passes runs bubble perm[t]
     uint32_t *cflag;   // connection bits, one per list entry
     const float4 *p0;
+    uint32_t step;     // 1, 2, .. within a run enqueued at once; 0: a query's pass
     float flag_sq;     // squared displacement from p0 beyond which the next step rebuilds (< 0: always)
 };
 
 // compute_forces + the integration of step (foam_dynamics.rs:62-94, 172-202); with force_out set,
 // only the forces of the current state.
 //
-// L lanes per bubble (L = 1 for large foams, where one thread per bubble already fills the GPU;
-// 4 or 16 for small ones, which would otherwise leave most SMs idle): the lanes evaluate the pair
-// forces of L consecutive list entries at once, then every lane of the group adds the L results
-// into the sum one by one in list order (shuffles), the buoyancy before the first j > k: the
-// reference's sums, the same on every lane; the group's first lane writes.
+// L lanes per bubble. The reference adds the pair forces in list order, the buoyancy before the first
+// j > k: that is one more list entry here, at `split`. The lanes evaluate kPair entries each, the next
+// ones' positions on the way, and put the forces in shared memory, from which each of three lanes sums
+// one component in order (entries past the list add zero, which changes no sum: none is ever -0).
+// Bound by instruction issue (78 % of the slots): 40000 bubbles take 101 us at four lanes; with four
+// IEEE divisions and a root per pair, shuffles between the lanes and every lane adding all the
+// components 271 us, 48 % issue, waiting for the positions.
+constexpr int kPair = 2;
 template <int L>
-__global__ void __launch_bounds__(kThreads, 5) forces_kernel(DynArgs a) {
+struct Exchange {
+    static constexpr int comp = L * kPair;                               // entries at once
+    static constexpr int group = 3 * comp + L;                            // no two groups on the same banks
+    static constexpr int warp = (32 / L) * group;
+};
+constexpr int kForceThreads = 128;
+
+template <int L>
+__global__ void __launch_bounds__(kForceThreads, 8) forces_kernel(DynArgs a) {
+    using X = Exchange<L>;
+    __shared__ __align__(16) float s_force[kForceThreads / 32][2][X::warp];
     Ctl *c = a.ctl;
-    if (c->fault != kFaultNone) return;
+    if (c->fault != kFaultNone || c->stale < a.step) return;
     const uint32_t n = c->n[a.npar];
     const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t t0 = gtid / L;
     const int sub = (int)(gtid % L);
     const int lane0 = (int)(threadIdx.x & 31) - sub;
-    const unsigned gmask = L == 32 ? 0xffffffffu : (((1u << L) - 1u) << lane0);
     if (gtid == 0 && !a.force_out) {
         c->steps_done += 1;
         c->nconn = 0;
         c->coal_key = kNoPair;
         c->merged_a = c->merged_b = kNone;
     }
-    if (t0 >= n) return;  // the whole group: t0 is the group's
-    const uint32_t k = a.perm[t0];
+    if ((gtid & ~31u) / L >= n) return;  // the whole warp
+    const bool live = t0 < n;
+    const uint32_t k = a.perm[live ? t0 : 0];
     const Phys &P = a.P;
     const float4 me = a.pr_in[k];
     const float4 mv = a.vt_in[k];
@@ -650,70 +706,61 @@ __global__ void __launch_bounds__(kThreads, 5) forces_kernel(DynArgs a) {
         by = ny * net;
         bz = nz * net;
     }
-    // entries t < split are j < k, whose pair force is evaluated with j first and enters negated;
-    // the buoyancy enters before the first j > k
-    float fx = 0.0f, fy = 0.0f, fz = 0.0f;
-    const uint32_t m = a.cnt[k], split = a.split[k];
-    const uint32_t *col = a.nbr + a.goff[t0 >> 5] + (t0 & 31);
-    if constexpr (L == 1) {
-        // one loop over the sorted list; the next entry's position fetched one iteration ahead
-        float4 next = m ? a.pr_in[__ldg(col)] : me;
-        for (uint32_t t = 0; t < m; ++t) {
-            const float4 o = next;
-            if (t + 1 < m) next = a.pr_in[__ldg(col + (size_t)(t + 1) * 32)];
-            if (t == split) {
-                fx = fx + bx;
-                fy = fy + by;
-                fz = fz + bz;
-            }
-            const bool lower = t < split;
-            float gx, gy, gz;
-            pair_force(P, lower ? o : me, lower ? me : o, gx, gy, gz);
-            fx = fx + (lower ? -gx : gx);
-            fy = fy + (lower ? -gy : gy);
-            fz = fz + (lower ? -gz : gz);
-        }
-    } else {
-        for (uint32_t base = 0; base < m; base += L) {
-            const uint32_t t = base + sub;
-            float gx = 0.0f, gy = 0.0f, gz = 0.0f;
-            if (t < m) {
-                const float4 o = a.pr_in[__ldg(col + (size_t)t * 32)];
-                const bool lower = t < split;
-                pair_force(P, lower ? o : me, lower ? me : o, gx, gy, gz);
-            }
-            const uint32_t cnt = min((uint32_t)L, m - base);  // the same on every lane of the group
+    // entries v < split are j < k, split is the buoyancy, the j > k follow, m is the last
+    const uint32_t split = live ? a.split[k] : 0u;
+    const uint32_t m = live ? a.cnt[k] : 0u;
+    const uint32_t *col = a.nbr + a.goff[(live ? t0 : 0u) >> 5] + (t0 & 31);
+    const auto index = [&](uint32_t v) {  // the bubble itself (whose force on itself is zero) where there is none
+        return v <= m && v != split ? __ldg(col + (size_t)(v - (v > split)) * 32) : k;
+    };
+    const uint32_t vmax = __reduce_max_sync(0xffffffffu, m);
+    uint32_t nj[kPair];
+    float4 next[kPair];
 #pragma unroll
-            for (int jj = 0; jj < L; ++jj) {
-                const float hx = __shfl_sync(gmask, gx, lane0 + jj);
-                const float hy = __shfl_sync(gmask, gy, lane0 + jj);
-                const float hz = __shfl_sync(gmask, gz, lane0 + jj);
-                if ((uint32_t)jj < cnt) {
-                    const uint32_t tt = base + jj;
-                    if (tt == split) {
-                        fx = fx + bx;
-                        fy = fy + by;
-                        fz = fz + bz;
-                    }
-                    const bool lower = tt < split;
-                    fx = fx + (lower ? -hx : hx);
-                    fy = fy + (lower ? -hy : hy);
-                    fz = fz + (lower ? -hz : hz);
-                }
+    for (int u = 0; u < kPair; ++u) next[u] = a.pr_in[index(u * L + sub)];
+#pragma unroll
+    for (int u = 0; u < kPair; ++u) nj[u] = index((kPair + u) * L + sub);
+    float fx = 0.0f;  // the sum of this lane's component
+    int buf = 0;
+    for (uint32_t base = 0; base <= vmax; base += X::comp) {
+        float g[3][kPair];
+#pragma unroll
+        for (int u = 0; u < kPair; ++u) {
+            const float4 o = next[u];
+            next[u] = a.pr_in[nj[u]];
+            nj[u] = index(base + (2 * kPair + u) * L + sub);
+            const uint32_t v = base + u * L + sub;
+            pair_force_near(P, me, o, v < split, g[0][u], g[1][u], g[2][u]);
+            if (v == split) {
+                g[0][u] = bx;
+                g[1][u] = by;
+                g[2][u] = bz;
             }
         }
+        float *row = s_force[threadIdx.x >> 5][buf] + (lane0 / L) * X::group;
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+            for (int u = 0; u < kPair; ++u) row[d * X::comp + u * L + sub] = g[d][u];
+        __syncwarp();  // the other buffer's readers have all passed the last one
+        const float4 *mine = reinterpret_cast<const float4 *>(row + min(sub, 2) * X::comp);
+#pragma unroll
+        for (int e = 0; e < X::comp / 4; ++e) {
+            const float4 q = mine[e];
+            fx = fx + q.x;
+            fx = fx + q.y;
+            fx = fx + q.z;
+            fx = fx + q.w;
+        }
+        buf ^= 1;
     }
-    if (split == m) {
-        fx = fx + bx;
-        fy = fy + by;
-        fz = fz + bz;
-    }
+    float fy = __shfl_sync(0xffffffffu, fx, lane0 + 1), fz = __shfl_sync(0xffffffffu, fx, lane0 + 2);
+    if (!live || sub != 0) return;
     // compute_drag (foam_dynamics.rs:163-167)
     const float drag_coeff = 6.0f * kPi * P.viscosity * me.w;
     fx = fx + (-mv.x) * drag_coeff;
     fy = fy + (-mv.y) * drag_coeff;
     fz = fz + (-mv.z) * drag_coeff;
-    if (sub != 0) return;
     if (a.force_out) {
         a.force_out[3 * (size_t)k] = fx;
         a.force_out[3 * (size_t)k + 1] = fy;
@@ -741,7 +788,7 @@ __global__ void __launch_bounds__(kThreads, 5) forces_kernel(DynArgs a) {
     // the neighbour list's displacement check on the new position (see connections_kernel)
     const float4 q0 = a.p0[k];
     const float ddx = np_.x - q0.x, ddy = np_.y - q0.y, ddz = np_.z - q0.z;
-    if (ddx * ddx + ddy * ddy + ddz * ddz > a.flag_sq) atomicOr(&c->need_rebuild, 1u);
+    if (ddx * ddx + ddy * ddy + ddz * ddz > a.flag_sq) atomicMin(&c->stale, a.step);
 }
 
 // update_connections (foam.rs:322-364) on the new positions: a bit per list entry j > i; with
@@ -753,27 +800,33 @@ __global__ void __launch_bounds__(kThreads, 5) forces_kernel(DynArgs a) {
 // build. The force pass flags a rebuild once a new position is within one step's travel
 // (v_max |dt|) of 0.45 skin, so the positions of the next step, which this pass and the next force
 // pass read, are still covered.
+//
+// A block per group of 32 bubbles: a lane per bubble, so that the columns are read whole, and the
+// words of flags dealt to the warps. With a thread per bubble 40000 of them left most of the GPU idle
+// and each walked its list alone.
 __global__ void __launch_bounds__(kThreads) connections_kernel(DynArgs a) {
     Ctl *c = a.ctl;
-    if (c->fault != kFaultNone) return;
+    if (c->fault != kFaultNone || c->stale < a.step) return;
     const uint32_t n = c->n[a.npar];
-    const uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t pos = blockIdx.x * 32 + (threadIdx.x & 31);
     uint32_t count = 0;
     if (pos < n) {
         const uint32_t i = a.perm[pos];
         const Phys &P = a.P;
         const float4 me = a.pr_out[i];
         const float4 mv = a.vt_out[i];
-        const uint32_t m = a.cnt[i], t0 = a.split[i];
+        const uint32_t m = a.cnt[i], t0 = a.split[i];  // the entries j > i: t0 and on
         const size_t g0 = a.goff[pos >> 5];
         const uint32_t *col = a.nbr + g0 + (pos & 31);
         uint32_t *fcol = a.cflag + (g0 >> 5) + (pos & 31);
         const float threshold = -me.w * 0.3f;
         bool want = P.coalescence != 0;
-        uint32_t word = 0;
-        for (uint32_t t = t0; t < m; ++t) {  // the entries j > i
-            const uint32_t j = __ldg(col + (size_t)t * 32);
-            {
+        for (uint32_t w = (t0 >> 5) + (threadIdx.x >> 5); w * 32 < m; w += kThreads / 32) {
+            uint32_t word = 0;
+            const uint32_t end = min(w * 32 + 32, m);
+#pragma unroll 4
+            for (uint32_t t = max(w * 32, t0); t < end; ++t) {
+                const uint32_t j = __ldg(col + (size_t)t * 32);
                 const float4 o = a.pr_out[j];
                 const float overlap = me.w + o.w - len3(me.x - o.x, me.y - o.y, me.z - o.z);
                 if (overlap > threshold) {
@@ -787,19 +840,15 @@ __global__ void __launch_bounds__(kThreads) connections_kernel(DynArgs a) {
                         const float4 ov = a.vt_out[j];
                         const float rel = (ov.x - mv.x) * nx + (ov.y - mv.y) * ny + (ov.z - mv.z) * nz;
                         const float weber = P.density * (rel * rel) * me.w / P.surface_tension;
-                        if (weber > P.coal_threshold) {
+                        if (weber > P.coal_threshold) {  // the smallest key is the first of all threads' firsts
                             atomicMin(&c->coal_key, ((unsigned long long)i << 32) | j);
                             want = false;
                         }
                     }
                 }
             }
-            if ((t & 31) == 31) {
-                fcol[(size_t)(t >> 5) * 32] = word;
-                word = 0;
-            }
+            fcol[(size_t)w * 32] = word;
         }
-        if (m & 31) fcol[(size_t)(m >> 5) * 32] = word;
     }
     for (int o = 16; o; o >>= 1) count += __shfl_xor_sync(0xffffffffu, count, o);
     if ((threadIdx.x & 31) == 0 && count) atomicAdd(&c->nconn, count);
@@ -809,7 +858,7 @@ __global__ void __launch_bounds__(kThreads) connections_kernel(DynArgs a) {
 // appends the merged one; copies the state unchanged when nothing merges.
 __global__ void __launch_bounds__(kThreads) merge_kernel(DynArgs a) {
     Ctl *c = a.ctl;
-    if (c->fault != kFaultNone) return;
+    if (c->fault != kFaultNone || c->stale < a.step) return;
     const uint32_t n = c->n[a.npar];
     const unsigned long long key = c->coal_key;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -847,7 +896,7 @@ __global__ void __launch_bounds__(kThreads) merge_kernel(DynArgs a) {
         c->merged_a = a.id_in[ia];
         c->merged_b = a.id_in[ib];
         c->n[a.npar ^ 1] = n - 1;
-        c->need_rebuild = 1;
+        atomicMin(&c->stale, a.step);
     }
 }
 
@@ -970,6 +1019,8 @@ struct sbs_foam_sim {
     Bufs b{};
     int cur = 0, npar = 0, conn_buf = 0, conn_npar = 0;
     bool list_invalid = true, stepped = false;
+    bool list_stale = false;  // the last step flagged a rebuild
+    uint32_t quiet = 32;      // steps to enqueue at once: twice what the last list served
     bool conn_cached = false;  // connections of the last step kept on the host (see sbs_foam_sim_forces)
     std::vector<sbs_bubble_connection> conn_cache;
     float list_skin = -1.0f;  // skin of the current neighbour list
@@ -1094,19 +1145,25 @@ DynArgs dyn_args(sbs_foam_sim *s, float dt, int in, int out) {
     a.nbr = s->nbr;
     a.cflag = s->cflag;
     a.p0 = s->p0;
+    a.step = 0;
     a.flag_sq = flag_sq_for(s->list_skin, dt);
     return a;
 }
 
-// Lanes per bubble of the force pass: enough threads to fill the GPU's SMs for small foams.
+constexpr uint32_t kLongestRun = 256, kEagerRun = 16;
+
+// Lanes per bubble of the force pass. More lanes fill the GPU where bubbles are few (and shorten the
+// walk of a list), but every lane of a group adds all its forces. us per step, launches included, at
+// 4 / 8 / 16 lanes: 1000 bubbles 73 / 67 / 59, 10000 95 / 80 / 80, 40000 135 / 128 / 157,
+// 80000 200 / 204 / 265, 200000 420 / 433 / 591 (one lane: 447, slower at every size).
 void launch_forces(sbs_foam_sim *s, const DynArgs &a) {
     const uint32_t n = s->n_cap;
-    if (n >= 131072)
-        forces_kernel<1><<<blocks(n), kThreads, 0, s->stream>>>(a);
-    else if (n >= 32768)
-        forces_kernel<4><<<blocks((size_t)n * 4), kThreads, 0, s->stream>>>(a);
+    if (n >= 65536)
+        forces_kernel<4><<<blocks((size_t)n * 4, kForceThreads), kForceThreads, 0, s->stream>>>(a);
+    else if (n >= 10000)
+        forces_kernel<8><<<blocks((size_t)n * 8, kForceThreads), kForceThreads, 0, s->stream>>>(a);
     else
-        forces_kernel<16><<<blocks((size_t)n * 16), kThreads, 0, s->stream>>>(a);
+        forces_kernel<16><<<blocks((size_t)n * 16, kForceThreads), kForceThreads, 0, s->stream>>>(a);
 }
 
 void free_list(sbs_foam_sim *s) {
@@ -1284,6 +1341,7 @@ int sbs_foam_sim_create(uint32_t n, const float *position, const float *radius, 
     c.next_id = n;
     c.coal_key = kNoPair;
     c.merged_a = c.merged_b = kNone;
+    c.stale = kNone;
     e = cudaMemcpyAsync(s->b.pr[0], pr.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, s->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(s->b.vt[0], vt.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, s->stream);
     if (e == cudaSuccess)
@@ -1316,18 +1374,30 @@ int sbs_foam_sim_step(sbs_foam_sim *s, float dt, uint32_t steps) {
     uint32_t done = 0;
     while (done < steps) {
         int rc;
-        if (s->list_invalid && (rc = rebuild_now(s, skin))) return rc;
+        if (s->list_invalid) {
+            if ((rc = rebuild_now(s, skin))) return rc;
+        } else if (s->list_stale) {
+            enqueue_list(s, true, skin);
+        }
+        s->list_stale = false;
+        // The steps of a run are enqueued at once; they read the list's state on the device. A step
+        // after which the list no longer holds stops the run: the later ones do nothing, and the next
+        // run starts with a rebuild. Enqueued before every step instead, a rebuild that has nothing to
+        // do is 13 launches, 50 us where the forces of 40000 bubbles take 100; that pays only where
+        // every step needs one (it saves the wait at the end of the run).
+        const bool eager = s->quiet <= 1;
+        const uint32_t run = std::min(steps - done, eager ? kEagerRun : s->quiet);
         const int cur0 = s->cur, npar0 = s->npar;
         SBS_CUDA_TRY(cudaMemsetAsync(&s->ctl->steps_done, 0, sizeof(uint32_t), s->stream));
-        for (uint32_t k = done; k < steps; ++k) {
-            enqueue_list(s, false, skin);
+        for (uint32_t k = 0; k < run; ++k) {
+            if (eager && k) enqueue_list(s, false, skin);
             DynArgs a = dyn_args(s, dt, s->cur, s->cur ^ 1);
+            a.step = k + 1;
             launch_forces(s, a);
-            if (coal || k + 1 == steps) connections_kernel<<<blocks(s->n_cap), kThreads, 0, s->stream>>>(a);
-            s->conn_buf = s->cur ^ 1;
-            s->conn_npar = s->npar;
+            if (coal || done + k + 1 == steps) connections_kernel<<<blocks(s->n_cap, 32), kThreads, 0, s->stream>>>(a);
             if (coal) {
                 DynArgs m = dyn_args(s, dt, s->cur ^ 1, s->cur);
+                m.step = k + 1;
                 merge_kernel<<<blocks(s->n_cap), kThreads, 0, s->stream>>>(m);
                 s->npar ^= 1;
             } else {
@@ -1338,10 +1408,8 @@ int sbs_foam_sim_step(sbs_foam_sim *s, float dt, uint32_t steps) {
         Ctl h;
         if ((rc = read_ctl(s, &h))) return rc;
         s->stepped = true;
-        if (h.fault == kFaultNone) break;
         if (h.fault == kFaultWalk) return set_error(SBS_E_STATE, "foam neighbour list: walk and count passes disagree");
-        // The list outgrew its storage at a rebuild: the steps from there on did nothing. Restore
-        // the buffer parities of the last completed step, grow the list and continue.
+        // the buffer parities of the last completed step
         done += h.steps_done;
         if (coal) {
             s->cur = cur0;
@@ -1353,6 +1421,15 @@ int sbs_foam_sim_step(sbs_foam_sim *s, float dt, uint32_t steps) {
             s->conn_buf = s->cur;
             s->conn_npar = s->npar;
         }
+        s->list_stale = h.stale != kNone;
+        if (h.fault == kFaultNone) {
+            if (eager) s->quiet = 2;  // see whether it is still so
+            else if (s->list_stale) s->quiet = std::min(2 * h.steps_done - (h.steps_done == 1), kLongestRun);
+            else if (run == s->quiet) s->quiet = std::min(2 * run, kLongestRun);
+            continue;
+        }
+        // The list outgrew its storage at a rebuild: the steps from there on did nothing. Grow it and
+        // continue.
         if (h.fault == kFaultDense)
             return set_error(SBS_E_INVALID,
                              "foam too dense: bubble %u has %u neighbours within 3 (r_a + r_b) + skin (limit %d)",
@@ -1490,7 +1567,7 @@ int sbs_foam_sim_forces(sbs_foam_sim *s, float *forces, int mem) {
     } else {
         Ctl h;
         if ((rc = read_ctl(s, &h))) return rc;
-        if (h.need_rebuild) {
+        if (h.stale != kNone) {
             // the rebuild overwrites the list that the last step's connections are read from: keep
             // them on the host first
             if (s->stepped && !s->conn_cached) {
@@ -1502,6 +1579,7 @@ int sbs_foam_sim_forces(sbs_foam_sim *s, float *forces, int mem) {
                 s->conn_cached = true;
             }
             enqueue_list(s, false, s->list_skin);
+            s->list_stale = false;
         }
     }
     uint32_t n = 0;
@@ -1538,7 +1616,7 @@ int sbs_foam_sim_connections(sbs_foam_sim *s, sbs_bubble_connection *out, uint32
         SBS_CUDA_TRY(cudaMemsetAsync(&s->ctl->merged_a, 0xff, 2 * sizeof(uint32_t), s->stream));
         DynArgs a = dyn_args(s, 0.0f, s->cur, s->cur);
         a.P.coalescence = 0;
-        connections_kernel<<<blocks(s->n_cap), kThreads, 0, s->stream>>>(a);
+        connections_kernel<<<blocks(s->n_cap, 32), kThreads, 0, s->stream>>>(a);
         SBS_CUDA_TRY(cudaGetLastError());
         s->conn_buf = s->cur;
         s->conn_npar = s->npar;

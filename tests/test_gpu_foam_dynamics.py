@@ -199,3 +199,46 @@ def test_bad_arguments(fd, sbs):
     sim = fd.FoamSimulator.with_default_cluster()
     with pytest.raises(sbs.SbsError):
         sim.step(float("inf"))
+
+
+@pytest.mark.parametrize("n", [1, 31, 9_999, 10_000, 10_001, 65_535, 65_537])
+def test_lanes_per_bubble_edges(fd, orc, n):
+    """The sizes where the lanes per bubble change, and groups that do not fill a warp."""
+    pos, rad = fd.fcc_foam(n, seed=41)
+    sim = fd.FoamSimulator(pos, rad)
+    idx = np.unique(np.concatenate([[0, n - 1], np.random.default_rng(42).integers(0, n, 24)]))
+    np.testing.assert_array_equal(sim.compute_forces()[idx], orc.foam_forces_subset(sim.physics, pos, rad, idx))
+
+
+@pytest.mark.parametrize("case", ["tiny offsets", "tiny strength", "no strength", "negative strength", "huge strength",
+                                  "huge radii", "tiny radii"])
+def test_pair_force_outside_ordinary_ranges(fd, orc, case):
+    """Where the shared reciprocal's residuals would not be exact the operators are used."""
+    pos, rad = fd.fcc_foam(200, seed=51)
+    kw = {"tiny strength": {"van_der_waals_strength": 1e-26}, "no strength": {"van_der_waals_strength": 0.0},
+          "negative strength": {"van_der_waals_strength": -0.002},
+          "huge strength": {"van_der_waals_strength": 1e25}}.get(case, {})
+    if case == "tiny offsets":  # a sheet of bubbles a few 1e-30 off its plane
+        pos = np.array(pos)
+        pos[:, 1] = np.random.default_rng(52).normal(0, 1, 200) * 10.0 ** np.random.default_rng(53).uniform(-38, -25, 200)
+    scale = {"huge radii": 1e17, "tiny radii": 1e-5}.get(case, 1.0)
+    pos, rad = (np.asarray(pos) * scale).astype(np.float32), (np.asarray(rad) * scale).astype(np.float32)
+    p = _phys(fd, **kw)
+    sim = fd.FoamSimulator(pos, rad, physics=p)
+    np.testing.assert_array_equal(sim.compute_forces(), orc.foam_forces(p, pos, rad))
+
+
+@pytest.mark.parametrize("dt,calls", [(1e-4, [70]), (5e-3, [45, 3, 1, 40]), (0.02, [10, 1, 1, 7]), (0.016, [1, 33, 2])])
+def test_runs_of_steps_match_oracle(fd, orc, dt, calls):
+    """Calls longer than a run enqueued at once, runs stopped by a list that no longer holds, and lists
+    rebuilt at every step, in a row of calls with a force query in between."""
+    pos, rad = fd.fcc_foam(400, seed=61)
+    sim = fd.FoamSimulator(pos, rad)
+    done = 0
+    for k in calls:
+        sim.step(dt, k)
+        done += k
+        want = orc.foam_step(sim.physics, dt, done, pos, rad)
+        _same_state(sim, want)
+        np.testing.assert_array_equal(sim.compute_forces(), orc.foam_forces(sim.physics, want["position"], want["radius"],
+                                                                            velocity=want["velocity"]))
