@@ -15,13 +15,14 @@
 // BF16 contraction).
 //
 // Spectrum generation: sin(phase/2) with phase = 2 pi opd/lambda + pi equals cos(pi y), y =
-// opd/lambda; cos^2 has period 1 in y, so y is reduced exactly to u = y - rint(y) in [-1/2, 1/2]
-// and cos(pi u) is the Taylor series of cos up to u^14 (truncation < 1e-8 on that interval; FP32
+// opd/lambda; cos^2 has period 1 in y, so y is reduced to u = y - rint(y) in [-1/2, 1/2] (rint by
+// adding and taking off 1.5 * 2^23 for |y| < 2^21, rintf beyond) and cos(pi u) is the Taylor series of cos up to u^14 (truncation < 1e-8 on that interval; FP32
 // mode) or up to u^8 (< 2.6e-5; the BF16 tensor-core mode, whose spectra are rounded to BF16),
 // evaluated two wavelengths at a time with packed FP32 instructions.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -45,6 +46,7 @@ struct BTile {
 struct SpecConsts {
     float invl[kMaxLambda];     // 1 / lambda (nm^-1), zero beyond nl
     float cmf[kMaxLambda][3];   // FP32 colour-matching weights (FP32 mode)
+    float invl_max;             // the largest of invl
     int nl;
 };
 
@@ -74,15 +76,28 @@ __device__ __forceinline__ float2 cos_pi_u2_short(float2 v) {
 
 // Airy reflectance F s^2 / (1 + F s^2) at two wavelengths (interference_lut.rs:123-133); SHORT:
 // the u^8 cosine series (BF16 spectra).
-template <bool SHORT = false>
+template <bool SHORT, bool FAR>
 __device__ __forceinline__ float2 airy2(float opd, float F, float il0, float il1) {
-    const float2 y = mul2(f2(opd), make_float2(il0, il1));
-    const float2 u = sub2(y, make_float2(rintf(y.x), rintf(y.y)));
+    const float2 il = make_float2(il0, il1);
+    float2 u;
+    if (FAR) {
+        const float2 y = mul2(f2(opd), il);
+        u = sub2(y, make_float2(rintf(y.x), rintf(y.y)));
+    } else {
+        const float2 y = make_float2(__fmul_rn(opd, il.x), __fmul_rn(opd, il.y));  // not part of an FMA
+        u = add2(y, fma2(add2(y, f2(12582912.0f)), f2(-1.0f), f2(12582912.0f)));
+    }
     const float2 c = SHORT ? cos_pi_u2_short(mul2(u, u)) : cos_pi_u2(mul2(u, u));
     const float2 fs = mul2(f2(F), mul2(c, c));
     const float2 den = add2(f2(1.0f), fs);
-    return make_float2(__fdividef(fs.x, den.x), __fdividef(fs.y, den.y));
+    float2 q;  // den >= 1: an ulp or so off, as __fdividef, without its care for denormal operands
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q.x) : "f"(den.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q.y) : "f"(den.y));
+    return mul2(fs, q);
 }
+
+// Whether |opd| / lambda stays below 2^21 for every wavelength (not for NaN).
+__device__ __forceinline__ bool opd_near(float opd, const SpecConsts &c) { return fabsf(opd) * c.invl_max < 2097152.0f; }
 
 // Per-point Snell / Fresnel / optical path (interference_lut.rs:54-61, 96-120 and the finesse F).
 __device__ __forceinline__ void point_setup(float t, float ci, float nf, float &F, float &opd) {
@@ -136,25 +151,44 @@ __device__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, long long limit
     return true;
 }
 
-// Writes one point's spectrum (row `row` of an A tile) as KPAD BF16 values.
+// Writes one point's spectrum (row `row` of an A tile) as KPAD BF16 values, zeros beyond nl. Groups of
+// eight wavelengths are evaluated without a branch between them, so that their chains overlap.
 template <int KPAD>
 __device__ __forceinline__ void write_spectrum_row(uint8_t *sA, int row, float opd, float F, const SpecConsts &c) {
     constexpr uint32_t SBO = (KPAD / 8) * 128;
+    const auto pack = [](float2 v) {
+        __nv_bfloat162 b2 = __floats2bfloat162_rn(v.x, v.y);
+        return *reinterpret_cast<uint32_t *>(&b2);
+    };
+    const bool near = opd_near(opd, c);
+    if (near) {
 #pragma unroll
-    for (int k8 = 0; k8 < KPAD; k8 += 8) {
-        uint32_t w[4];
+        for (int k8 = 0; k8 < KPAD; k8 += 8) {
+            uint32_t w[4] = {0u, 0u, 0u, 0u};
+            if (k8 + 8 <= c.nl) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int l = k8 + 2 * j;
-            float2 v = make_float2(0.f, 0.f);  // padding beyond nl: zeros, not evaluated
-            if (l < c.nl) {
-                v = airy2<true>(opd, F, c.invl[l], c.invl[l + 1]);
-                if (l + 1 >= c.nl) v.y = 0.f;
+                for (int j = 0; j < 4; ++j)
+                    w[j] = pack(airy2<true, false>(opd, F, c.invl[k8 + 2 * j], c.invl[k8 + 2 * j + 1]));
+            } else if (k8 < c.nl) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int l = k8 + 2 * j;
+                    if (l >= c.nl) break;
+                    float2 v = airy2<true, false>(opd, F, c.invl[l], c.invl[l + 1]);
+                    if (l + 1 >= c.nl) v.y = 0.f;
+                    w[j] = pack(v);
+                }
             }
-            __nv_bfloat162 b2 = __floats2bfloat162_rn(v.x, v.y);
-            w[j] = *reinterpret_cast<uint32_t *>(&b2);
+            *reinterpret_cast<uint4 *>(sA + tile_off(row, k8, SBO)) = make_uint4(w[0], w[1], w[2], w[3]);
         }
-        *reinterpret_cast<uint4 *>(sA + tile_off(row, k8, SBO)) = make_uint4(w[0], w[1], w[2], w[3]);
+    } else {
+#pragma unroll 1
+        for (int l = 0; l < KPAD; l += 2) {
+            float2 v = make_float2(0.f, 0.f);
+            if (l < c.nl) v = airy2<true, true>(opd, F, c.invl[l], c.invl[l + 1]);
+            if (l + 1 >= c.nl) v.y = 0.f;
+            *reinterpret_cast<uint32_t *>(sA + tile_off(row, l, SBO)) = pack(v);
+        }
     }
 }
 
@@ -290,19 +324,23 @@ __global__ void __launch_bounds__(128) spectral_fp32_kernel(const float *__restr
     float F, opd;
     point_setup(t_nm[p], cos_i[p], n_film[p], F, opd);
     float r = 0.f, g = 0.f, b = 0.f;
-#pragma unroll
-    for (int l = 0; l < KPAD; l += 2) {
-        if (l < c.nl) {
-            const float2 v = airy2(opd, F, c.invl[l], c.invl[l + 1]);
-            r = fmaf(v.x, c.cmf[l][0], r);
-            g = fmaf(v.x, c.cmf[l][1], g);
-            b = fmaf(v.x, c.cmf[l][2], b);
-            if (l + 1 < c.nl) {
-                r = fmaf(v.y, c.cmf[l + 1][0], r);
-                g = fmaf(v.y, c.cmf[l + 1][1], g);
-                b = fmaf(v.y, c.cmf[l + 1][2], b);
-            }
+    const auto add = [&](int l, float2 v) {
+        r = fmaf(v.x, c.cmf[l][0], r);
+        g = fmaf(v.x, c.cmf[l][1], g);
+        b = fmaf(v.x, c.cmf[l][2], b);
+        if (l + 1 < c.nl) {
+            r = fmaf(v.y, c.cmf[l + 1][0], r);
+            g = fmaf(v.y, c.cmf[l + 1][1], g);
+            b = fmaf(v.y, c.cmf[l + 1][2], b);
         }
+    };
+    if (opd_near(opd, c)) {
+#pragma unroll
+        for (int l = 0; l < KPAD; l += 2)
+            if (l < c.nl) add(l, airy2<false, false>(opd, F, c.invl[l], c.invl[l + 1]));
+    } else {
+#pragma unroll 1
+        for (int l = 0; l < c.nl; l += 2) add(l, airy2<false, true>(opd, F, c.invl[l], c.invl[l + 1]));
     }
     rgb[3 * p] = r;
     rgb[3 * p + 1] = g;
@@ -364,6 +402,7 @@ extern "C" int sbs_spectral_rgb(const float *t_nm, const float *cos_i, const flo
     for (uint32_t l = 0; l < nl; ++l) {
         SBS_CHECK_ARG(wl_nm[l] > 0.f, "wavelengths must be positive");
         c.invl[l] = 1.0f / wl_nm[l];
+        c.invl_max = std::max(c.invl_max, c.invl[l]);
         for (int ch = 0; ch < 3; ++ch) c.cmf[l][ch] = cmf[3 * l + ch];
     }
     const int kpad = nl <= 32 ? 32 : (nl <= 64 ? 64 : (nl <= 96 ? 96 : 128));

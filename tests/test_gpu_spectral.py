@@ -86,3 +86,19 @@ def test_spectral_very_thick_films(sbs, orc):
         assert rel_linf(got[thin], want) <= tol, mode
         g = got[thick]
         assert np.isfinite(g).all() and (g >= -1e-3).all() and (g <= cap * 1.01 + 1e-3).all(), mode
+
+
+@pytest.mark.parametrize("nl", [1, 8, 9, 81, 96, 127])
+@pytest.mark.parametrize("mode,bar", [("fp32", 1e-4), ("tc", 1e-2)])
+def test_partial_groups_of_wavelengths(sbs, orc, nl, mode, bar):
+    """Wavelength counts on both sides of a group of eight, with points of the far reduction (films
+    whose opd / lambda passes 2^21) in the same warps, which may not disturb their neighbours."""
+    t, c, nf, wl, cmf = workload(1000, seed=nl, nl=nl)
+    want = orc.spectral_rgb(t, c, nf, wl, cmf)
+    far = np.arange(5, 1000, 9)
+    t = t.copy()
+    t[far] = np.float32(1.2e9)
+    got = sbs.spectral_rgb(t, c, nf, wl, cmf, mode=mode)
+    near = np.setdiff1d(np.arange(1000), far)
+    assert np.max(np.abs(got[near] - want[near])) <= bar * np.max(np.abs(want))
+    assert np.isfinite(got).all() and (got >= -bar).all()
