@@ -2,7 +2,7 @@
 // the forward pass of layers 1-3 (pre-activations and activations kept for the backward pass) and
 // the input gradient of layers 2-3 (the transposed convolution times the activation's derivative).
 //
-// Work item: 16 output rows of one 128-cell column segment of one field; one CTA (8 warps) per
+// Work item: a few output rows (launch_tc: how many) of one 128-cell column segment of one field; one CTA (8 warps) per
 // item walks it top to bottom. Input rows are staged through a ring of five row buffers by
 // per-thread cp.async copies, three rows ahead of the row whose MMAs are issued, as planes of 8 channels with 16 bytes per cell (the K-major, no-swizzle layout of
 // an MMA's A operand: 8-cell core matrices 128 B apart, planes a plane apart), 130 cells wide (one
@@ -24,6 +24,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "nn.cuh"
 #include "nn_kernels.h"
 #include "sbs_internal.h"
@@ -38,7 +40,7 @@ constexpr int kTcCells = 128;                   // output cells per segment (MMA
 constexpr int kTcStage = kTcCells + 2;          // staged cells per input row
 constexpr uint32_t kTcPlane = kTcStage * 16;    // one 8-channel plane: 2080 B
 constexpr int kTcRing = 5;                      // input row buffers: rows r-1..r+1 read, r+2, r+3 landing
-constexpr int kTcRows = 16;                     // output rows per work item
+constexpr int kTcMaxRows = 64, kTcStart = 4;    // output rows per work item; what its start costs, in rows
 constexpr uint32_t kTcId = tc::idesc_bf16_m128(32);
 
 constexpr int kTcYS = 36;  // floats per cell in the FP32 tiles (32 + 4: conflict-free 16 B accesses)
@@ -71,7 +73,7 @@ struct TcConvArgs {
     bf16 *aout;           // forward: activations; transposed: gradient of the layer below
     unsigned *err;        // bit 1: a wait timed out
     long long wait_cycles;
-    int nt, np, segs, nrb, nitems;
+    int nt, np, segs, rows, nrb, nitems;  // rows: output rows per item
     int act;              // SBS_NN_ACT_*
     int stall;            // timeout test: issue neither MMAs nor commits
 };
@@ -126,7 +128,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_conv_kernel(const TcConvArgs a)
 
     for (int item = blockIdx.x; item < a.nitems && !failed; item += gridDim.x) {
         const int rb = item % a.nrb, seg = (item / a.nrb) % a.segs, f = item / (a.nrb * a.segs);
-        const int r0 = rb * kTcRows, r1 = min(nt, r0 + kTcRows);
+        const int r0 = rb * a.rows, r1 = min(nt, r0 + a.rows);
         const int j0 = seg * kTcCells;
         const bf16 *base = a.in + (size_t)f * nt * np * CIN;
         const size_t cell0 = (size_t)f * nt * np;
@@ -530,7 +532,26 @@ cudaError_t launch_tc(TcConvArgs a, int nf, cudaStream_t st) {
                                          (int)Lay::SMEM);
     if (e != cudaSuccess) return e;
     a.segs = (a.np + kTcCells - 1) / kTcCells;
-    a.nrb = (a.nt + kTcRows - 1) / kTcRows;
+    int dev = 0, sms = 1, smem_sm = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess) return e;
+    // Rows per item: the items run in rounds of as many as fit the GPU (by shared memory, 1 KB each
+    // reserved by the runtime), and the last round costs as much as a full one. Eight training steps of
+    // eight 256 x 512 fields take 7.6 ms with the 29 (32 input channels) and 19 (16) rows this picks,
+    // 8.1 with 16 rows for all (two rounds, the second two thirds full); four 512 x 1024 fields 26.2
+    // against 27.0, 128 x 256 2.9 against 3.3.
+    const long long slots = (long long)std::max(1, smem_sm / (int)(Lay::SMEM + 1024)) * sms;
+    long long best = 0;
+    for (int rows = 4; rows <= kTcMaxRows; ++rows) {
+        const long long items = (long long)nf * a.segs * ((a.nt + rows - 1) / rows);
+        const long long cost = (items + slots - 1) / slots * (rows + kTcStart);
+        if (best == 0 || cost < best) {
+            best = cost;
+            a.rows = rows;
+        }
+    }
+    a.nrb = (a.nt + a.rows - 1) / a.rows;
     a.nitems = nf * a.segs * a.nrb;
     const WaitConfig w = wait_config();
     a.wait_cycles = w.cycles;
