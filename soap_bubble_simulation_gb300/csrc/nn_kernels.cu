@@ -17,6 +17,7 @@
 #include "nn.cuh"
 #include "nn_kernels.h"
 #include "sbs_internal.h"
+#include "tc.cuh"
 
 namespace sbs {
 namespace nn {
@@ -58,224 +59,329 @@ struct OutArgs {
     int nf;
 };
 
-// The three source rows i - 1, i, i + 1 (theta reflected) of a3 for cells j0 - 1 .. j0 + 128 (phi
-// wrapped) into dst[row][cell][0..31], one 16-byte copy per thread and step. For rows of at least
-// 128 cells one correction wraps a column (the cells span less than two row lengths).
-constexpr int kSegCells = 128;  // cells per row segment of the layer-4 kernels
-template <int STRIDE>
-__device__ __forceinline__ void stage_rows3(bf16 (*dst)[kSegCells + 2][STRIDE], const bf16 *a3, size_t fb, int i,
-                                            int nt, int np, int j0) {
-    const int ru = refl_row(i - 1, nt), rd = refl_row(i + 1, nt);
-    const bool wide = np >= kSegCells;
-    for (int e = threadIdx.x; e < 3 * (kSegCells + 2) * 4; e += blockDim.x) {
-        const int d = e / ((kSegCells + 2) * 4), rem = e - d * ((kSegCells + 2) * 4), q = rem >> 2, ch = rem & 3;
-        int col = j0 - 1 + q;
-        if (wide) {
-            col = col < 0 ? col + np : (col >= np ? col - np : col);
-        } else {
-            col %= np;
-            col = col < 0 ? col + np : col;
+// The three layer-4 kernels walk columns: a warp takes a few adjacent columns (its lanes also divide
+// the 32 channels) of a strip of rows and goes down it, so the taps' weights or sums stay in
+// registers and a row's operands are read and widened once for the three rows they meet. They are
+// bound by the FP32 issue of 288 multiply-adds per cell (about 100 instructions per warp and row
+// against a row's loads); what ran before took a cell's nine taps from shared memory, 36 to 72 reads
+// and up to 288 conversions per cell. Eight 256 x 512 fields, microseconds before and now: output
+// layer 75 and 44, weight gradient 84 and 33, input gradient 68 and 57.
+//
+// Work is dealt as (field, strip, column group) units, groups fastest, to the warps of a grid that
+// fits the GPU. A strip's rows minimise the rounds of units times a unit's rows, kWalkExtra of which
+// stand for the two rows beyond the strip and the start of the pipeline.
+constexpr int kWalkWarps = 8, kWalkExtra = 4;
+struct Walk {
+    int rows, strips, groups, units, blocks;
+};
+
+inline cudaError_t plan_walk(int nf, int nt, int np, int cols, int blocks_per_sm, Walk *w) {
+    int dev = 0, sms = 1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    const long long groups = (np + cols - 1) / cols, warps = (long long)sms * blocks_per_sm * kWalkWarps;
+    long long best = 0;
+    for (int rows = 4; rows < nt + 4; rows += 4) {
+        const long long units = nf * groups * ((nt + rows - 1) / rows);
+        const long long cost = (units + warps - 1) / warps * (rows + kWalkExtra);
+        if (best == 0 || cost < best) {
+            best = cost;
+            w->rows = rows;
         }
-        const int r = d == 0 ? ru : (d == 1 ? i : rd);
-        *reinterpret_cast<uint4 *>(&dst[d][q][ch * 8]) =
-            *reinterpret_cast<const uint4 *>(a3 + (fb + (size_t)r * np + col) * 32 + ch * 8);
     }
+    w->strips = (nt + w->rows - 1) / w->rows;
+    w->groups = (int)groups;
+    w->units = nf * w->strips * w->groups;
+    w->blocks = (int)std::min<long long>((long long)sms * blocks_per_sm, (w->units + kWalkWarps - 1) / kWalkWarps);
+    return cudaSuccess;
 }
 
-// One block per item (an output row x a 128-cell segment): the three source rows of a3 (130 cells
-// each, phi wrapped, theta reflected) are staged in shared memory with 80 bytes per cell (16-byte
-// reads of consecutive cells fall in distinct banks), then one thread per cell. The four chunk sums
-// of a cell run as two packed FP32x2 pairs (chunks 0, 1 and 2, 3): each half performs its chunk's
-// multiply-adds tap by tap and channel by channel, so y is bitwise that of four scalar chains.
-constexpr int kOutCells = kSegCells;
-constexpr int kOutStride = 40;  // BF16 values per staged cell (32 + 8)
+// A warp's rows arrive through its own ring in shared memory, kWalkRing - 1 rows ahead by per-lane
+// cp.async: one row ahead in registers left the loads' latency uncovered (1,600 cycles a row where
+// 600 were issued).
+constexpr int kWalkRing = 8;
+__device__ __forceinline__ void walk_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kWalkRing - 2) : "memory"); }
 
-__global__ void __launch_bounds__(kOutCells, 7) out_kernel(OutArgs a) {  // 7 blocks: the shared-memory limit
-    __shared__ float2 swp[9][2][8];  // tap, chunk pair: (W4[tap][16 kp + c], W4[tap][16 kp + 8 + c])
-    __shared__ __align__(16) bf16 sa[3][kOutCells + 2][kOutStride];
-    __shared__ double sred[kOutCells / 32];
+// Two BF16 values of a word, widened.
+__device__ __forceinline__ float bf_lo(uint32_t u) { return __uint_as_float(u << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
+
+// Output layer: eight columns a warp, four lanes (8-channel chunks) a cell. Every source row adds
+// its nine taps to the three output rows it belongs to; an output row's chunk sums are complete,
+// tap by tap and channel by channel, when the row below it has been added. The lane of chunk k
+// finishes the strip's rows k, k + 4, ... (loss, gradient), so that work is done by all lanes.
+constexpr int kOutCols = 8, kOutBlocksPerSm = 2;  // two blocks: 72 weights and the rows in flight, 128 registers
+
+__global__ void __launch_bounds__(32 * kWalkWarps, kOutBlocksPerSm) out_kernel(OutArgs a, Walk k) {
+    __shared__ __align__(16) uint4 ring[kWalkWarps][kWalkRing][4 * (kOutCols + 2)];
+    __shared__ double sred[kWalkWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ch = lane & 3;
     const int nt = a.g.nt, np = a.g.np;
-    const int segs = (np + kOutCells - 1) / kOutCells;
-    const int row = (int)(blockIdx.x / segs), j0 = (int)(blockIdx.x % segs) * kOutCells;
-    const int i = row % nt;
-    const size_t fb = (size_t)(row / nt) * nt * np;
-    for (int e = threadIdx.x; e < 9 * 16; e += blockDim.x) {
-        const int t = e >> 4, kp = (e >> 3) & 1, c = e & 7;
-        swp[t][kp][c] = make_float2(a.w4[t * 32 + 16 * kp + c], a.w4[t * 32 + 16 * kp + 8 + c]);
+    float w[72];  // [tap][channel of the chunk]
+#pragma unroll
+    for (int t = 0; t < 9; ++t) {
+        const float4 *p = reinterpret_cast<const float4 *>(a.w4 + t * 32 + ch * 8);
+        const float4 u = p[0], v = p[1];
+        w[8 * t] = u.x, w[8 * t + 1] = u.y, w[8 * t + 2] = u.z, w[8 * t + 3] = u.w;
+        w[8 * t + 4] = v.x, w[8 * t + 5] = v.y, w[8 * t + 6] = v.z, w[8 * t + 7] = v.w;
     }
-    stage_rows3<kOutStride>(sa, a.a3, fb, i, nt, np, j0);
-    __syncthreads();
-    const int m = threadIdx.x, j = j0 + m;
+    const float b4 = *a.b4;
     double l = 0.0;
-    if (j < np) {
-        const size_t c = fb + (size_t)i * np + j;
-        // four independent partial sums (one per 8-channel chunk), as the pairs (0, 1) and (2, 3)
-        float2 y01 = make_float2(0.f, 0.f), y23 = y01;
-#pragma unroll
-        for (int t = 0; t < 9; ++t) {
-            const int d = t / 3, x = t % 3;  // source row i + d - 1 (reflected when staged), cell j + x - 1
-            const uint4 *p = reinterpret_cast<const uint4 *>(&sa[d][m + x][0]);
-            const uint4 v0 = p[0], v1 = p[1], v2 = p[2], v3 = p[3];
-            const uint32_t u0[4] = {v0.x, v0.y, v0.z, v0.w}, u1[4] = {v1.x, v1.y, v1.z, v1.w};
-            const uint32_t u2[4] = {v2.x, v2.y, v2.z, v2.w}, u3[4] = {v3.x, v3.y, v3.z, v3.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&u0[e]));
-                const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&u1[e]));
-                const float2 f2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&u2[e]));
-                const float2 f3 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&u3[e]));
-                y01 = __ffma2_rn(swp[t][0][2 * e], make_float2(f0.x, f1.x), y01);
-                y01 = __ffma2_rn(swp[t][0][2 * e + 1], make_float2(f0.y, f1.y), y01);
-                y23 = __ffma2_rn(swp[t][1][2 * e], make_float2(f2.x, f3.x), y23);
-                y23 = __ffma2_rn(swp[t][1][2 * e + 1], make_float2(f2.y, f3.y), y23);
+    for (int u = blockIdx.x * kWalkWarps + warp; u < k.units; u += gridDim.x * kWalkWarps) {
+        const int grp = u % k.groups, v = u / k.groups, f = v / k.strips, r0 = (v - f * k.strips) * k.rows;
+        const int r1 = min(nt, r0 + k.rows);
+        const int j0 = grp * kOutCols, jt = j0 + (lane >> 2);
+        const size_t fb = (size_t)f * nt * np;
+        const uint4 *src = reinterpret_cast<const uint4 *>(a.a3 + fb * 32);
+        // slot cells 0..9 are columns j0 - 1 .. j0 + 8, wrapped
+        const int ca = (j0 - 1 + (lane >> 2) + np) % np * 4 + ch, cb = (j0 + 7 + ((lane & 7) >> 2)) % np * 4 + ch;
+        auto fill = [&](int r) {
+            if (r <= r1) {
+                const uint4 *p = src + (size_t)refl_row(r, nt) * np * 4;
+                uint4 *dst = ring[warp][(r + 1) % kWalkRing];
+                tc::cp_async16(dst + lane, p + ca);
+                if (lane < 8) tc::cp_async16(dst + 32 + lane, p + cb);
             }
-        }
-        const float y = __fadd_rn(*a.b4, __fadd_rn(__fadd_rn(y01.x, y01.y), __fadd_rn(y23.x, y23.y)));
-        a.y4[c] = y;
-        if (a.target) {
-            const float mk = a.g.rows[i].w;
-            float gr = 0.f;
-            if (mk != 0.f) {
-                const float dd = __fsub_rn(y, a.target[c]);
-                l = (double)dd * (double)dd;
-                gr = __fmul_rn(dd, a.inv_nmask2);
+            tc::cp_async_commit();
+        };
+        __syncwarp();  // the previous unit's rows are read
+#pragma unroll
+        for (int d = 0; d < kWalkRing - 1; ++d) fill(r0 - 1 + d);
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f, mine = 0.f;  // rows r + 1, r, r - 1; the lane's finished row
+        for (int r = r0 - 1; r <= r1; ++r) {
+            walk_wait();
+            __syncwarp();  // row r is there, row r - 1 is read
+            fill(r + kWalkRing - 1);
+            const uint4 *row = ring[warp][(r + 1) % kWalkRing] + lane;
+            s2 = s1;
+            s1 = s0;
+            s0 = 0.f;
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                const uint4 now = row[4 * x];
+                const uint32_t q[4] = {now.x, now.y, now.z, now.w};
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const float v = c & 1 ? bf_hi(q[c >> 1]) : bf_lo(q[c >> 1]);
+                    s2 = __fmaf_rn(w[8 * (6 + x) + c], v, s2);
+                    s1 = __fmaf_rn(w[8 * (3 + x) + c], v, s1);
+                    s0 = __fmaf_rn(w[8 * x + c], v, s0);
+                }
             }
-            a.g4[c] = gr;
+            const int i = r - 1 - r0;  // the finished row in the strip
+            if (i < 0) continue;
+            float y = __fadd_rn(s2, __shfl_xor_sync(0xffffffffu, s2, 1));
+            y = __fadd_rn(b4, __fadd_rn(y, __shfl_xor_sync(0xffffffffu, y, 2)));
+            if ((i & 3) == ch) mine = y;
+            if ((i & 3) != 3 && r < r1) continue;
+            const int out = r0 + (i & ~3) + ch;
+            if (out >= r1 || jt >= np) continue;
+            const size_t c = fb + (size_t)out * np + jt;
+            a.y4[c] = mine;
+            if (a.target) {
+                float gr = 0.f;
+                if (a.g.rows[out].w != 0.f) {
+                    const float dd = __fsub_rn(mine, a.target[c]);
+                    l += (double)dd * (double)dd;
+                    gr = __fmul_rn(dd, a.inv_nmask2);
+                }
+                a.g4[c] = gr;
+            }
         }
     }
     if (a.target) {
         for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-        if ((threadIdx.x & 31) == 0) sred[threadIdx.x >> 5] = l;
+        if (lane == 0) sred[warp] = l;
         __syncthreads();
         if (threadIdx.x == 0) {
             double sum = 0.0;
-            for (int k = 0; k < kOutCells / 32; ++k) sum += sred[k];
+            for (int q = 0; q < kWalkWarps; ++q) sum += sred[q];
             a.loss_part[blockIdx.x] = sum;
         }
     }
 }
 
-// dW4[tap][ic] = sum g4[cell] a3[src(cell,tap)][ic], db4 = sum g4. Work item: one output row x one
-// 128-cell segment; block b takes items b, b + nblocks, ... Per item the block stages the three
-// source rows of a3 (130 cells each, phi wrapped, theta reflected) and the row's g4 in shared
-// memory; warp w sums the item's cells w, w + 8, ... with lane = ic and nine accumulators per lane
-// (one per tap). One partial row [289] per block, warps summed in a fixed order. An item's rows are
-// loaded and then used with nothing else in flight, so the grid is sized for six blocks per SM
-// (kW4BlocksPerSm): other blocks' loads cover each block's wait.
+// dW4[tap][ic] = sum g4[cell] a3[src(cell,tap)][ic], db4 = sum g4. Lanes as in the output layer; a
+// lane holds its chunk's 72 sums, and a source cell's eight channels meet the nine gradients of the
+// output cells that read it (three rows and columns, kept as the rows go by; zero outside the
+// strip). One partial row [289] per block: lanes, then warps, in a fixed order.
 struct Wgrad4Args {
     const float *g4;
     const bf16 *a3;
     float *partial;
     GridTab g;
-    int rows;  // fields x nt
 };
 
-constexpr int kW4Warps = 8;
-constexpr int kW4Cells = kSegCells;
-constexpr int kW4BlocksPerSm = 6;  // 34.7 KB of shared memory and 40 registers a thread each
+constexpr int kW4BlocksPerSm = 2;
 
-__global__ void __launch_bounds__(32 * kW4Warps, kW4BlocksPerSm) wgrad4_kernel(Wgrad4Args a) {
-    __shared__ __align__(16) bf16 sa[3][kW4Cells + 2][32];
-    __shared__ float sg[kW4Cells];
-    __shared__ float sp[kW4Warps][289];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+__global__ void __launch_bounds__(32 * kWalkWarps, kW4BlocksPerSm) wgrad4_kernel(Wgrad4Args a, Walk k) {
+    __shared__ __align__(16) uint4 ring[kWalkWarps][kWalkRing][4 * kOutCols];
+    __shared__ float gring[kWalkWarps][kWalkRing][12];
+    __shared__ float sp[kWalkWarps][289];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ch = lane & 3;
     const int nt = a.g.nt, np = a.g.np;
-    const int segs = (np + kW4Cells - 1) / kW4Cells, items = a.rows * segs;
-    float acc[9];
+    float acc[72];
 #pragma unroll
-    for (int t = 0; t < 9; ++t) acc[t] = 0.f;
+    for (int t = 0; t < 72; ++t) acc[t] = 0.f;
     float gsum = 0.f;
-    for (int item = blockIdx.x; item < items; item += gridDim.x) {
-        const int row = item / segs, j0 = (item % segs) * kW4Cells;
-        const int i = row % nt;
-        const size_t fb = (size_t)(row / nt) * nt * np;
-        const int n = min(kW4Cells, np - j0);
-        __syncthreads();  // the previous item's tiles are read
-        for (int e = tid; e < 3 * (kW4Cells + 2) * 4; e += blockDim.x) {
-            const int d = e / ((kW4Cells + 2) * 4), q = (e / 4) % (kW4Cells + 2), ch = e % 4;
-            int col = (j0 - 1 + q) % np;
-            col = col < 0 ? col + np : col;
-            const size_t src = (fb + (size_t)refl_row(i + d - 1, nt) * np + col) * 32 + ch * 8;
-            *reinterpret_cast<uint4 *>(&sa[d][q][ch * 8]) = *reinterpret_cast<const uint4 *>(a.a3 + src);
-        }
-        for (int e = tid; e < kW4Cells; e += blockDim.x) sg[e] = e < n ? a.g4[fb + (size_t)i * np + j0 + e] : 0.f;
-        __syncthreads();
-        for (int m = warp; m < n; m += kW4Warps) {
-            const float gv = sg[m];
-            if (lane == 0) gsum = __fadd_rn(gsum, gv);
+    for (int u = blockIdx.x * kWalkWarps + warp; u < k.units; u += gridDim.x * kWalkWarps) {
+        const int grp = u % k.groups, v = u / k.groups, f = v / k.strips, r0 = (v - f * k.strips) * k.rows;
+        const int r1 = min(nt, r0 + k.rows);
+        const int j0 = grp * kOutCols, n = min(kOutCols, np - j0), q = lane >> 2;
+        const size_t fb = (size_t)f * nt * np;
+        const uint4 *src = reinterpret_cast<const uint4 *>(a.a3 + fb * 32) + (size_t)min(j0 + q, np - 1) * 4 + ch;
+        // slot cells 0..9 are the gradients of columns j0 - 1 .. j0 + 8, wrapped
+        const float *gp = a.g4 + fb + (j0 - 1 + lane + np) % np;
+        auto fill = [&](int r) {  // source row r and the gradients of row r + 1 (zero outside the strip)
+            if (r <= r1) {
+                const int s = (r + 2) % kWalkRing;
+                tc::cp_async16_zfill(&ring[warp][s][lane], src + (size_t)refl_row(r, nt) * np * 4, q < n);
+                const bool ok = r + 1 >= r0 && r + 1 < r1;
+                if (lane < 10) tc::cp_async4_zfill(&gring[warp][s][lane], gp + (ok ? (size_t)(r + 1) * np : 0), ok);
+            }
+            tc::cp_async_commit();
+        };
+        __syncwarp();  // the previous unit's rows are read
 #pragma unroll
-            for (int d = 0; d < 3; ++d)
+        for (int d = 0; d < kWalkRing - 1; ++d) fill(r0 - 1 + d);
+        // tap (d, x) of output cell (i, q) reads source (i + d - 1, q + x - 1): g[d][x] is the gradient
+        // of row r - d + 1, column q - x + 1
+        float g[3][3];
 #pragma unroll
-                for (int x = 0; x < 3; ++x)
-                    acc[3 * d + x] = __fmaf_rn(gv, __bfloat162float(sa[d][m + x][lane]), acc[3 * d + x]);
+        for (int x = 0; x < 3; ++x) g[0][x] = g[1][x] = 0.f;
+        for (int r = r0 - 1; r <= r1; ++r) {
+            walk_wait();
+            __syncwarp();  // row r is there, row r - 1 is read
+            fill(r + kWalkRing - 1);
+            const int s = (r + 2) % kWalkRing;
+            const uint4 now = ring[warp][s][lane];
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                g[2][x] = g[1][x];
+                g[1][x] = g[0][x];
+                g[0][x] = gring[warp][s][q + 2 - x];
+            }
+            if (q < n) gsum = __fadd_rn(gsum, g[1][1]);
+            const uint32_t w[4] = {now.x, now.y, now.z, now.w};
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const float v = c & 1 ? bf_hi(w[c >> 1]) : bf_lo(w[c >> 1]);
+#pragma unroll
+                for (int t = 0; t < 9; ++t) acc[8 * t + c] = __fmaf_rn(g[t / 3][t % 3], v, acc[8 * t + c]);
+            }
         }
     }
 #pragma unroll
-    for (int t = 0; t < 9; ++t) sp[warp][t * 32 + lane] = acc[t];
+    for (int t = 0; t < 72; ++t) {
+        float v = acc[t];
+        for (int o = 4; o < 32; o <<= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
+        if (lane < 4) sp[warp][(t >> 3) * 32 + ch * 8 + (t & 7)] = v;
+    }
+    for (int o = 4; o < 32; o <<= 1) gsum = __fadd_rn(gsum, __shfl_xor_sync(0xffffffffu, gsum, o));
     if (lane == 0) sp[warp][288] = gsum;
     __syncthreads();
-    for (int k = tid; k < 289; k += blockDim.x) {
+    for (int e = threadIdx.x; e < 289; e += blockDim.x) {
         float v = 0.f;
-        for (int w = 0; w < kW4Warps; ++w) v = __fadd_rn(v, sp[w][k]);
-        a.partial[(size_t)blockIdx.x * 289 + k] = v;
+        for (int q = 0; q < kWalkWarps; ++q) v = __fadd_rn(v, sp[q][e]);
+        a.partial[(size_t)blockIdx.x * 289 + e] = v;
     }
 }
 
 // g3[cell][ic] = bf16( (sum over the taps that read `cell` of g4[out] W4[tap][ic]) * act'(y3) ):
-// one thread per cell with its 32 channels in registers (taps in the order t = 0..8, each tap's
-// pole-reflection source right after its own term).
+// four columns a warp, eight lanes (4 channels) a cell, so that a warp's y3 and g3 accesses are
+// whole 128-byte lines (a thread per cell, 128 bytes apart, kept the L1 busy for 40 of 68 us). Taps
+// in the order t = 0..8, each tap's pole-reflection source right after its own term.
 struct Dgrad4Args {
     const float *g4;
     const float *w4;
     const float *y3;
     bf16 *g3;
     GridTab g;
-    size_t cells;
     int act;  // SBS_NN_ACT_*
 };
 
-__global__ void __launch_bounds__(256) dgrad4_kernel(Dgrad4Args a) {
-    __shared__ float sw[288];
-    for (int k = threadIdx.x; k < 288; k += blockDim.x) sw[k] = a.w4[k];
-    __syncthreads();
-    const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= a.cells) return;
+constexpr int kD4Cols = 4, kD4BlocksPerSm = 3;
+
+__global__ void __launch_bounds__(32 * kWalkWarps, kD4BlocksPerSm) dgrad4_kernel(Dgrad4Args a, Walk k) {
+    __shared__ __align__(16) float4 ring[kWalkWarps][kWalkRing][8 * kD4Cols];
+    __shared__ float gring[kWalkWarps][kWalkRing][8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ch = lane & 7;
     const int nt = a.g.nt, np = a.g.np;
-    const int j = (int)(c % np), i = (int)((c / np) % nt);
-    const size_t fb = (c / ((size_t)np * nt)) * nt * np;
-    float s[32];
-#pragma unroll
-    for (int ic = 0; ic < 32; ++ic) s[ic] = 0.f;
+    float2 w[9][2];
 #pragma unroll
     for (int t = 0; t < 9; ++t) {
-        const int dy = t / 3 - 1, dx = t % 3 - 1;
-        const int r = i - dy;
-        int q = j - dx;
-        q = q < 0 ? q + np : (q >= np ? q - np : q);
-        const float gm = r >= 0 && r < nt ? a.g4[fb + (size_t)r * np + q] : 0.f;
-        const bool xt = i == 1 && dy == -1, xb = i == nt - 2 && dy == 1;
-        const float ge = xt ? a.g4[fb + q] : xb ? a.g4[fb + (size_t)(nt - 1) * np + q] : 0.f;
-        const bool has_m = r >= 0 && r < nt;
-#pragma unroll
-        for (int ic = 0; ic < 32; ++ic) {
-            if (has_m) s[ic] = __fmaf_rn(gm, sw[t * 32 + ic], s[ic]);
-            if (xt || xb) s[ic] = __fmaf_rn(ge, sw[t * 32 + ic], s[ic]);
-        }
+        const float4 u = *reinterpret_cast<const float4 *>(a.w4 + t * 32 + ch * 4);
+        w[t][0] = make_float2(u.x, u.y);
+        w[t][1] = make_float2(u.z, u.w);
     }
-    const float4 *yp = reinterpret_cast<const float4 *>(a.y3 + c * 32);
-    uint4 *gp = reinterpret_cast<uint4 *>(a.g3 + c * 32);
+    for (int u = blockIdx.x * kWalkWarps + warp; u < k.units; u += gridDim.x * kWalkWarps) {
+        const int grp = u % k.groups, v = u / k.groups, f = v / k.strips, r0 = (v - f * k.strips) * k.rows;
+        const int r1 = min(nt, r0 + k.rows);
+        const int j0 = grp * kD4Cols, q = lane >> 3, j = min(j0 + q, np - 1);
+        const size_t fb = (size_t)f * nt * np;
+        const float4 *yp = reinterpret_cast<const float4 *>(a.y3 + fb * 32) + (size_t)j * 8 + ch;
+        uint2 *op = reinterpret_cast<uint2 *>(a.g3 + (fb + (size_t)r0 * np) * 32) + (size_t)j * 8 + ch;
+        // slot cells 0..5 are the gradients of columns j0 - 1 .. j0 + 4, wrapped
+        const float *gp = a.g4 + fb + (j0 - 1 + lane + np) % np;
+        auto fill = [&](int r) {  // row r of y3 (from r0 on) and the gradients of row r + 1
+            if (r < r1) {
+                const int s = (r + 2) % kWalkRing;
+                if (r >= r0) tc::cp_async16(&ring[warp][s][lane], yp + (size_t)r * np * 8);
+                if (lane < 6)
+                    tc::cp_async4_zfill(&gring[warp][s][lane], gp + (size_t)min(max(r + 1, 0), nt - 1) * np, true);
+            }
+            tc::cp_async_commit();
+        };
+        __syncwarp();  // the previous unit's rows are read
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float4 y0 = yp[2 * k], y1 = yp[2 * k + 1];
-        const float v[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
-        uint32_t w[4];
+        for (int d = 0; d < kWalkRing - 1; ++d) fill(r0 - 2 + d);
+        // tap (dy, dx) reads the gradient of cell (r - dy, j - dx): g[0] is row r + 1, g[2] row r - 1
+        float g[3][3];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 g = __fmul2_rn(make_float2(s[8 * k + 2 * e], s[8 * k + 2 * e + 1]),
-                                        act_grad2(a.act, make_float2(v[2 * e], v[2 * e + 1])));
-            w[e] = pack2(g.x, g.y);
+        for (int x = 0; x < 3; ++x) g[0][x] = g[1][x] = 0.f;
+        for (int r = r0 - 2; r < r1; ++r) {
+            walk_wait();
+            __syncwarp();  // row r is there, row r - 1 is read
+            fill(r + kWalkRing - 1);
+            const int sl = (r + 2) % kWalkRing;
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                g[2][x] = g[1][x];
+                g[1][x] = g[0][x];
+                g[0][x] = gring[warp][sl][q + 2 - x];
+            }
+            if (r < r0) continue;
+            const float4 y = ring[warp][sl][lane];
+            float2 s[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+            if (r >= 2 && r + 2 < nt) {
+#pragma unroll
+                for (int t = 0; t < 9; ++t) {
+                    const float2 m = make_float2(g[t / 3][t % 3], g[t / 3][t % 3]);
+                    s[0] = __ffma2_rn(m, w[t][0], s[0]);
+                    s[1] = __ffma2_rn(m, w[t][1], s[1]);
+                }
+            } else {  // the rows next to a pole: no row beyond it, the pole's own row reflected into 1 and nt - 2
+#pragma unroll
+                for (int t = 0; t < 9; ++t) {
+                    const bool own = t < 3 ? r + 1 < nt : t < 6 || r >= 1;
+                    const bool top = r == 1 && t < 3, bottom = r == nt - 2 && t >= 6;
+                    const float m = g[t / 3][t % 3], e = g[2 - t / 3][t % 3];
+                    if (own) {
+                        s[0] = __ffma2_rn(make_float2(m, m), w[t][0], s[0]);
+                        s[1] = __ffma2_rn(make_float2(m, m), w[t][1], s[1]);
+                    }
+                    if (top || bottom) {
+                        s[0] = __ffma2_rn(make_float2(e, e), w[t][0], s[0]);
+                        s[1] = __ffma2_rn(make_float2(e, e), w[t][1], s[1]);
+                    }
+                }
+            }
+            const float2 u0 = __fmul2_rn(s[0], act_grad2(a.act, make_float2(y.x, y.y)));
+            const float2 u1 = __fmul2_rn(s[1], act_grad2(a.act, make_float2(y.z, y.w)));
+            if (j0 + q < np) *op = make_uint2(pack2(u0.x, u0.y), pack2(u1.x, u1.y));
+            op += (size_t)np * 8;
         }
-        gp[k] = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
@@ -471,30 +577,30 @@ cudaError_t output_layer(const bf16 *a3, const Packed &p, float *y4, const float
     o.g = g;
     o.nf = nf;
     o.b4 = p.b + 96;
-    const int nb = nf * g.nt * ((g.np + kOutCells - 1) / kOutCells);  // one block per row segment
-    out_kernel<<<nb, kOutCells, 0, st>>>(o);
-    if (nblocks_out) *nblocks_out = nb;
+    Walk k{};
+    const cudaError_t e = plan_walk(nf, g.nt, g.np, kOutCols, kOutBlocksPerSm, &k);
+    if (e != cudaSuccess) return e;
+    out_kernel<<<k.blocks, 32 * kWalkWarps, 0, st>>>(o, k);
+    if (nblocks_out) *nblocks_out = k.blocks;
     return cudaGetLastError();
 }
 
 cudaError_t output_backward(const float *g4, const bf16 *a3, const float *y3, const Packed &p, bf16 *g3,
-                            float *partial, int nblocks, float *grad, const GridTab &g, int nf, cudaStream_t st) {
-    const size_t cells = (size_t)nf * g.nt * g.np;
+                            float *partial, float *grad, const GridTab &g, int nf, cudaStream_t st) {
     Wgrad4Args w{};
     w.g4 = g4;
     w.a3 = a3;
     w.partial = partial;
     w.g = g;
-    w.rows = nf * g.nt;
-    // nblocks is two per SM (the 3x3 layers' partial rows); six per SM here, whose rows of 289
-    // floats fit the same buffer of nblocks x (32 x 9 x 32 + 32) floats
-    static_assert(kW4BlocksPerSm * 289 <= 2 * (32 * 9 * 32 + 32), "layer-4 partial rows fit the buffer");
-    const int nb4 = nblocks / 2 * kW4BlocksPerSm;
-    wgrad4_kernel<<<nb4, 32 * kW4Warps, 0, st>>>(w);
-    cudaError_t e = cudaGetLastError();
+    Walk k{};
+    cudaError_t e = plan_walk(nf, g.nt, g.np, kOutCols, kW4BlocksPerSm, &k);
     if (e != cudaSuccess) return e;
-    reduce4_kernel<<<(289 + kRedCols - 1) / kRedCols, kRedCols * kRed4Rows, 0, st>>>(partial, nb4, grad + SBS_NN_W4,
-                                                                                  grad + SBS_NN_B4);
+    // partial rows of 289 floats in a buffer of nblocks (two per SM) x (32 x 9 x 32 + 32) floats
+    static_assert(kW4BlocksPerSm * 289 <= 2 * (32 * 9 * 32 + 32), "layer-4 partial rows fit the buffer");
+    wgrad4_kernel<<<k.blocks, 32 * kWalkWarps, 0, st>>>(w, k);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    reduce4_kernel<<<(289 + kRedCols - 1) / kRedCols, kRedCols * kRed4Rows, 0, st>>>(
+        partial, k.blocks, grad + SBS_NN_W4, grad + SBS_NN_B4);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     Dgrad4Args d{};
     d.g4 = g4;
@@ -502,9 +608,9 @@ cudaError_t output_backward(const float *g4, const bf16 *a3, const float *y3, co
     d.y3 = y3;
     d.g3 = g3;
     d.g = g;
-    d.cells = cells;
     d.act = p.act;
-    dgrad4_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>(d);
+    if ((e = plan_walk(nf, g.nt, g.np, kD4Cols, kD4BlocksPerSm, &k)) != cudaSuccess) return e;
+    dgrad4_kernel<<<k.blocks, 32 * kWalkWarps, 0, st>>>(d, k);
     return cudaGetLastError();
 }
 

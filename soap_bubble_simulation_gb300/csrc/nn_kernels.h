@@ -38,7 +38,7 @@ cudaError_t output_layer(const bf16 *a3, const Packed &p, float *y4, const float
                          double *loss_part, float inv_nmask2, const GridTab &g, int nf, cudaStream_t st,
                          int *nblocks_out);
 cudaError_t output_backward(const float *g4, const bf16 *a3, const float *y3, const Packed &p, bf16 *g3,
-                            float *partial, int nblocks, float *grad, const GridTab &g, int nf, cudaStream_t st);
+                            float *partial, float *grad, const GridTab &g, int nf, cudaStream_t st);
 cudaError_t adam(float *theta, float *m, float *v, const float *grad, float lr, float b1, float b2, float eps,
                  int step, cudaStream_t st);
 cudaError_t pack(const float *theta, const Packed &p, cudaStream_t st);

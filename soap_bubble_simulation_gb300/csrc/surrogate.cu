@@ -260,7 +260,7 @@ int loss_and_grad(sbs_surrogate *s, const Fields &fs, int nf, const GridDev &g, 
     int nlb = 0;
     SBS_CUDA_TRY(output_layer(s->a3, s->pk, s->y4, s->tgt, s->g4, s->loss_part, (float)(2.0 / nmask), g.tab(), nf,
                               s->stream, &nlb));
-    SBS_CUDA_TRY(output_backward(s->g4, s->a3, s->y3, s->pk, s->g3, s->partial, s->nblocks, s->grad, g.tab(), nf,
+    SBS_CUDA_TRY(output_backward(s->g4, s->a3, s->y3, s->pk, s->g3, s->partial, s->grad, g.tab(), nf,
                                  s->stream));
     SBS_CUDA_TRY(conv_backward_weight(3, s->g3, s->a2, s->partial, s->nblocks, s->grad, s->pk.err, nf, nt, np,
                                       s->stream));

@@ -1,5 +1,5 @@
 // Small wrappers of the Blackwell tensor-core (tcgen05), mbarrier, TMA and cp.async instructions used
-// by the surrogate's training convolutions (nn_conv_tc.cu).
+// by the surrogate's training kernels (nn_conv_tc.cu, nn_kernels.cu).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -119,6 +119,15 @@ __device__ __forceinline__ void pin(uint32_t &r) { asm volatile("" : "+r"(r)); }
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
+}
+// 16 or 4 bytes, zeros where !valid (nothing is read then)
+__device__ __forceinline__ void cp_async16_zfill(void *smem, const void *gmem, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(smem)), "l"(gmem), "r"(valid ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async4_zfill(void *smem, const void *gmem, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(smem_u32(smem)), "l"(gmem), "r"(valid ? 4 : 0)
+                 : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }

@@ -107,6 +107,25 @@ def test_gradients_match_oracle(sbs, orc, net, nt, np_, nf):
         assert e <= 3e-2, (name, e)
 
 
+# The layer-4 kernels go down strips of rows, 8 or 4 columns a warp. 5 x 9: one strip longer than the
+# grid, a column beyond a group of 8 and of 4; 7 x 131: two strips, the last of three rows; 118 x 515:
+# strips of several groups of four rows, a ragged last one; 4 x 1224 with 16 fields: the most fields,
+# more units than warps.
+@pytest.mark.parametrize("nt,np_,nf", [(5, 9, 1), (7, 131, 2), (118, 515, 2), (4, 1224, 16)])
+def test_layer4_strips_match_oracle(sbs, orc, net, nt, np_, nf):
+    h, c = fields(nf, nt, np_, seed=13)
+    ps = params_list(sbs, nf, nt, np_, seed=14)
+    target = np.random.default_rng(15).standard_normal((nf, nt, np_)).astype(np.float32)
+    x = np.stack([orc.nn_features(h[b], c[b], orc_params(orc, ps[b])) for b in range(nf)])
+    check_y(net.forward(h, c, ps, mode="layered"), orc.nn_forward(net.params, x, net.activation))
+    loss, grad = net.loss_grad(h, c, ps, target)
+    loss_o, grad_o = orc.nn_loss_grad(net.params, x, target, net.activation)
+    assert abs(loss - loss_o) <= 1e-3 * loss_o
+    for name, a, b in LAYERS:
+        e = np.abs(grad[a:b] - grad_o[a:b]).max() / np.abs(grad_o[a:b]).max()
+        assert e <= 3e-2, (name, e)
+
+
 def trained_surrogate(sbs, ntraj=24, nt=48, np_=96, iters=300, activation="gelu"):
     s = sbs.DrainageSurrogate(seed=3, activation=activation)
     g = np.random.default_rng(0)
