@@ -2,16 +2,19 @@
 // the forward pass of layers 1-3 (pre-activations and activations kept for the backward pass) and
 // the input gradient of layers 2-3 (the transposed convolution times the activation's derivative).
 //
-// Work item: a few output rows (launch_tc: how many) of one 128-cell column segment of one field; one CTA (8 warps) per
-// item walks it top to bottom. Input rows are staged through a ring of five row buffers by
-// per-thread cp.async copies, three rows ahead of the row whose MMAs are issued, as planes of 8 channels with 16 bytes per cell (the K-major, no-swizzle layout of
-// an MMA's A operand: 8-cell core matrices 128 B apart, planes a plane apart), 130 cells wide (one
-// halo cell each side, phi wrapped). The dx = -1 / 0 / +1 taps read the same buffer at start
+// Work item: a few output rows (launch_tc: how many) of one 128-cell column segment of one field; one
+// CTA (8 warps) per item walks it top to bottom. Input rows are staged through a ring of five row
+// buffers by per-thread cp.async copies, three rows ahead of the row whose MMAs are issued, as planes
+// of 8 channels with 16 bytes per cell (the K-major, no-swizzle layout of an MMA's A operand: 8-cell
+// core matrices 128 B apart, planes a plane apart), 130 cells wide (one halo cell each side, phi
+// wrapped). The dx = -1 / 0 / +1 taps read the same buffer at start
 // addresses 16 bytes apart, so there is no im2col copy. One output row is 9 taps x CIN/16 MMAs of
 // M = 128 cells x N = 32 channels x K = 16 into a 32-column TMEM accumulator; two accumulators
 // alternate, so the epilogue of row r - 1 (tcgen05.ld, bias and activation, or the activation's
 // derivative, and the stores) runs while the MMAs of row r execute. The weights are staged once per
-// CTA as the B operand (32 rows of 16-byte K chunks).
+// CTA as the B operand (32 rows of 16-byte K chunks). Bound by the epilogue's issue and by waits: a
+// row had three block barriers, of which one is left (the warps' epilogues are their own). Eight
+// 256 x 512 fields, microseconds before and now: layers 2 and 3 forward 88 and 72, transposed 89 and 65.
 //
 // theta: the forward pass reflects at the poles (source row -1 is row 1, row nt is row nt-2); the
 // transposed pass reads the gradient at row i - dy, skips rows outside the grid, and adds the
@@ -49,6 +52,7 @@ constexpr int kTcAS = 40;  // BF16 values per cell in the output tile (32 + 8)
 template <int CIN, bool BWD>
 struct TcLayout {
     static constexpr int PL = CIN / 8;                   // planes per input row
+    static constexpr int PIECES = (kTcStage * PL + kTcThreads - 1) / kTcThreads;  // staged per thread and row
     static constexpr uint32_t ROWB = PL * kTcPlane;      // bytes per staged row
     static constexpr int KC = CIN / 16;                  // K16 steps per tap
     static constexpr uint32_t BCH = 32 * 16;             // one 8-element K chunk of B (32 rows)
@@ -123,7 +127,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_conv_kernel(const TcConvArgs a)
     uint64_t b_desc[9 * Lay::KC];
 #pragma unroll
     for (int i = 0; i < 9 * Lay::KC; ++i) b_desc[i] = tc::make_desc(sb + Lay::OFF_B + (uint32_t)i * Lay::BSTEP, Lay::BCH, 128);
-    uint32_t issued[2] = {0u, 0u};  // commits on each barrier so far (block-uniform)
+    uint32_t issued0 = 0u, issued1 = 0u;  // commits on each barrier so far (block-uniform)
     bool failed = false;
 
     for (int item = blockIdx.x; item < a.nitems && !failed; item += gridDim.x) {
@@ -133,15 +137,21 @@ __global__ void __launch_bounds__(kTcThreads) tc_conv_kernel(const TcConvArgs a)
         const bf16 *base = a.in + (size_t)f * nt * np * CIN;
         const size_t cell0 = (size_t)f * nt * np;
 
+        // the thread's 16-byte pieces of a staged row: where in the row (phi wrapped), where in its buffer
+        int from[Lay::PIECES], to[Lay::PIECES];
+#pragma unroll
+        for (int i = 0; i < Lay::PIECES; ++i) {
+            const int e = tid + i * kTcThreads, q = e / Lay::PL, p = e % Lay::PL;
+            from[i] = (j0 - 1 + q + np) % np * CIN + p * 8;
+            to[i] = p * kTcPlane + q * 16;
+        }
         auto stage = [&](int r) {  // input row r into buffer r mod kTcRing (all threads)
             uint8_t *dst = smem + (r % kTcRing) * Lay::ROWB;
             const bf16 *rowp = base + (size_t)r * np * CIN;
-            for (int e = tid; e < kTcStage * Lay::PL; e += kTcThreads) {
-                const int q = e / Lay::PL, p = e % Lay::PL;
-                int col = (j0 - 1 + q) % np;
-                col = col < 0 ? col + np : col;
-                tc::cp_async16(dst + p * kTcPlane + q * 16, rowp + (size_t)col * CIN + p * 8);
-            }
+#pragma unroll
+            for (int i = 0; i < Lay::PIECES; ++i)
+                if ((i + 1) * kTcThreads <= kTcStage * Lay::PL || tid + i * kTcThreads < kTcStage * Lay::PL)
+                    tc::cp_async16(dst + to[i], rowp + from[i]);
         };
         auto issue = [&](int r, uint32_t dacc) {  // the MMAs of output row r (one thread)
             // buffers of rows r - 1, r, r + 1 in 16-byte units of the A descriptor's address field
@@ -174,22 +184,29 @@ __global__ void __launch_bounds__(kTcThreads) tc_conv_kernel(const TcConvArgs a)
             }
         };
         const int nvalid = min(kTcCells, np - j0);  // cells of the segment inside the grid
-        // transposed: pre-activations of output row r into tile (r - r0) & 1, 16 B per copy
+        // transposed: pre-activations of output row r into tile (r - r0) & 1, 16 B per copy; a warp
+        // fetches what its own epilogue reads (its 32 cells' 16 channels)
+        const int m0 = quarter * 32, c0 = 16 * half;
         auto prefetch_y = [&](int r) {
-            float *dst = s_y + ((r - r0) & 1) * kTcCells * kTcYS;
-            const float *src = a.yprev + (cell0 + (size_t)r * np + j0) * 32;
-            for (int e = tid; e < nvalid * 8; e += kTcThreads)
-                tc::cp_async16(dst + (e >> 3) * kTcYS + (e & 7) * 4, src + (size_t)e * 4);
+            float *dst = s_y + (((r - r0) & 1) * kTcCells + m0) * kTcYS + c0;
+            const float *src = a.yprev + (cell0 + (size_t)r * np + j0 + m0) * 32 + c0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int q = 8 * k + (lane >> 2), ch = (lane & 3) * 4;
+                if (m0 + q < nvalid) tc::cp_async16(dst + q * kTcYS + ch, src + q * 32 + ch);
+            }
         };
         // output row r from accumulator columns col..col+31: each thread its cell's 16 channels into
-        // the shared tiles, then the block copies the row out in contiguous 16-byte pieces
+        // the shared tiles, then the warp copies them out in 16-byte pieces (whole 32-byte sectors).
+        // Only the warp itself reads what it wrote, so a row has no block barrier but the one that
+        // ends its iteration.
         auto epilogue = [&](int r, uint32_t col) {
             uint32_t v[16];
             tc::tld16(tl + col, v);
             tc::wait_ld();
 #pragma unroll
             for (int k = 0; k < 16; ++k) tc::pin(v[k]);
-            const int m = quarter * 32 + lane, c0 = 16 * half;
+            const int m = m0 + lane;
             uint4 *ap = reinterpret_cast<uint4 *>(s_a + m * kTcAS + c0);
             if (!BWD) {
                 float y[16];
@@ -226,22 +243,29 @@ __global__ void __launch_bounds__(kTcThreads) tc_conv_kernel(const TcConvArgs a)
                     ap[k] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
                 }
             }
-            __syncthreads();
-            const size_t cb = cell0 + (size_t)r * np + j0;
-            uint4 *ga = reinterpret_cast<uint4 *>(a.aout + cb * 32);
-            for (int e = tid; e < nvalid * 4; e += kTcThreads)
-                ga[e] = *reinterpret_cast<const uint4 *>(s_a + (e >> 2) * kTcAS + (e & 3) * 8);
-            if (!BWD) {
-                float4 *gy = reinterpret_cast<float4 *>(a.yout + cb * 32);
-                for (int e = tid; e < nvalid * 8; e += kTcThreads)
-                    gy[e] = *reinterpret_cast<const float4 *>(s_y + (e >> 3) * kTcYS + (e & 7) * 4);
+            __syncwarp();
+            const size_t cb = (cell0 + (size_t)r * np + j0 + m0) * 32 + c0;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int q = 16 * k + (lane >> 1), ch = (lane & 1) * 8;
+                if (m0 + q < nvalid)
+                    *reinterpret_cast<uint4 *>(a.aout + cb + q * 32 + ch) =
+                        *reinterpret_cast<const uint4 *>(s_a + (m0 + q) * kTcAS + c0 + ch);
             }
+            if (!BWD) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int q = 8 * k + (lane >> 2), ch = (lane & 3) * 4;
+                    if (m0 + q < nvalid)
+                        *reinterpret_cast<float4 *>(a.yout + cb + q * 32 + ch) =
+                            *reinterpret_cast<const float4 *>(s_y + (m0 + q) * kTcYS + c0 + ch);
+                }
+            }
+            __syncwarp();
         };
-        // block-uniform: every thread waits for the same completion; the block agrees on the outcome
-        auto wait_acc = [&](int b) -> bool {
-            const bool ok = tc::mbar_wait_n(bar0 + 8u * b, issued[b] - 1u, a.wait_cycles);
-            return __syncthreads_or(ok ? 0 : 1) == 0;
-        };
+        // every thread waits for the same completion; the block agrees on the outcome at the
+        // iteration's end, and until then a thread whose wait ran out touches nothing
+        auto wait_acc = [&](int b) { return tc::mbar_wait_n(bar0 + 8u * b, (b ? issued1 : issued0) - 1u, a.wait_cycles); };
 
         const int rlast = min(nt - 1, r1);  // the last input row the item reads
         for (int r = max(0, r0 - 1); r <= min(rlast, r0 + 2); ++r) stage(r);
@@ -261,37 +285,33 @@ __global__ void __launch_bounds__(kTcThreads) tc_conv_kernel(const TcConvArgs a)
                 }
                 __syncwarp();
             }
-            ++issued[b];
-            if (r > r0) {
-                if (!wait_acc(b ^ 1)) {
-                    failed = true;
-                    break;
-                }
-                tc::fence_after();
-            }
+            b ? ++issued1 : ++issued0;
+            const bool ok = r == r0 || wait_acc(b ^ 1);
+            tc::fence_after();
             // row r + 3 replaces row r - 2, whose last reader (output row r - 1) has completed; it is
             // needed one iteration later, so only row r + 2 must have landed at this iteration's end
             // (one copy group per iteration, possibly empty)
-            if (r + 3 <= rlast) stage(r + 3);
-            if (r > r0) epilogue(r - 1, 32u * (b ^ 1));
-            // transposed: y of row r + 1 into the tile the epilogue above has finished reading
-            if (BWD && r + 1 < r1) prefetch_y(r + 1);
+            if (ok && r + 3 <= rlast) stage(r + 3);
+            if (__all_sync(0xffffffffu, ok)) {
+                if (r > r0) epilogue(r - 1, 32u * (b ^ 1));
+                // transposed: y of row r + 1 into the tile the epilogue above has finished reading
+                if (BWD && r + 1 < r1) prefetch_y(r + 1);
+            }
             tc::cp_async_commit();
             asm volatile("cp.async.wait_group 1;\n" ::: "memory");
             tc::fence_async_smem();
             tc::fence_before();
-            __syncthreads();
+            failed = __syncthreads_or(ok ? 0 : 1) != 0;
             tc::fence_after();
+            if (failed) break;
         }
         if (failed) break;
-        if (!wait_acc((r1 - 1 - r0) & 1)) {
-            failed = true;
-            break;
-        }
+        const int last = (r1 - 1 - r0) & 1;
+        const bool ok = wait_acc(last);
         tc::fence_after();
-        epilogue(r1 - 1, 32u * ((r1 - 1 - r0) & 1));
+        if (__all_sync(0xffffffffu, ok)) epilogue(r1 - 1, 32u * last);
         tc::fence_before();
-        __syncthreads();
+        failed = __syncthreads_or(ok ? 0 : 1) != 0;
         tc::fence_after();
     }
     if (failed) {
@@ -301,7 +321,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_conv_kernel(const TcConvArgs a)
             atomicOr(a.err, 2u);
             if (!a.stall)
                 for (int b = 0; b < 2; ++b)
-                    if (issued[b]) tc::mbar_wait_n(bar0 + 8u * b, issued[b] - 1u, a.wait_cycles);
+                    if (const uint32_t n = b ? issued1 : issued0) tc::mbar_wait_n(bar0 + 8u * b, n - 1u, a.wait_cycles);
         }
     }
     tc::cp_async_wait_all();
