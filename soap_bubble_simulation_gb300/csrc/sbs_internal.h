@@ -236,6 +236,8 @@ struct sbs_drainage {
     int x2 = 0;                          // 1: compensated f32x2 thickness
     int cur = 0;   // buffer index holding the newest field
     int prev = 1;  // buffer holding the field one pass older (WGSL quirk accessor)
+    void *small = nullptr;   // device memory of the small buffers below, but vol_out and qbuf
+    void *pinned = nullptr;  // host memory of sched_host and ring_status
     sbs::FixSum *part[2] = {nullptr, nullptr};  // per-block pole-ring partials (single-step kernel)
     float4 *rows = nullptr;
     double *vol_w = nullptr;
