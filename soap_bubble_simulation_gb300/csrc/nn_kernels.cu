@@ -434,10 +434,26 @@ __global__ void __launch_bounds__(kRedCols *kRed4Rows) reduce4_kernel(const floa
         *grad_b4 = s;
 }
 
-__global__ void adam_kernel(float *theta, float *m, float *v, const float *grad, int n, float lr, float b1,
-                            float b2, float eps, float c1, float c2) {
+// A step that may not be taken (a non-finite loss, a timed-out wait, a step before it that failed) is
+// decided here, so that the host need not read the loss before it enqueues the update and what
+// follows: every block sums the loss partials, in one fixed order, and comes to the same answer.
+// The first block records it for the host and for the steps behind it.
+__global__ void __launch_bounds__(256) adam_kernel(float *theta, float *m, float *v, const float *grad, int n, float lr,
+                                                   float b1, float b2, float eps, float c1, float c2, StepGate gate) {
+    __shared__ double part[256];
+    double sum = 0.0;
+    for (int k = threadIdx.x; k < gate.nparts; k += 256) sum += gate.parts[k];
+    part[threadIdx.x] = sum;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+        if (threadIdx.x < o) part[threadIdx.x] += part[threadIdx.x + o];
+        __syncthreads();
+    }
+    const double loss = part[0] / gate.nmask;
+    const unsigned code = gate.prev && gate.prev->code ? gate.prev->code : *gate.err ? 2u : isfinite(loss) ? 0u : 1u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *gate.log = StepLog{loss, code, 0u};
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n) return;
+    if (e >= n || code) return;
     const float g = grad[e];
     const float mm = b1 * m[e] + (1.f - b1) * g;
     const float vv = b2 * v[e] + (1.f - b2) * g * g;
@@ -615,11 +631,11 @@ cudaError_t output_backward(const float *g4, const bf16 *a3, const float *y3, co
 }
 
 cudaError_t adam(float *theta, float *m, float *v, const float *grad, float lr, float b1, float b2, float eps,
-                 int step, cudaStream_t st) {
+                 int step, const StepGate &gate, cudaStream_t st) {
     const float c1 = (float)(1.0 / (1.0 - std::pow((double)b1, step)));
     const float c2 = (float)(1.0 / (1.0 - std::pow((double)b2, step)));
     adam_kernel<<<(SBS_NN_PARAMS + 255) / 256, 256, 0, st>>>(theta, m, v, grad, SBS_NN_PARAMS, lr, b1, b2, eps, c1,
-                                                             c2);
+                                                             c2, gate);
     return cudaGetLastError();
 }
 

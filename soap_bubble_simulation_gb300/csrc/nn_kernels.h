@@ -39,8 +39,24 @@ cudaError_t output_layer(const bf16 *a3, const Packed &p, float *y4, const float
                          int *nblocks_out);
 cudaError_t output_backward(const float *g4, const bf16 *a3, const float *y3, const Packed &p, bf16 *g3,
                             float *partial, float *grad, const GridTab &g, int nf, cudaStream_t st);
+// What one training step came to; code 1: the loss is not finite, 2: a wait timed out (of this step
+// or, either, of one before it in the run).
+struct StepLog {
+    double loss;
+    unsigned code, pad;
+};
+// What decides whether an update is made: the loss partials, the error word, the log of the step
+// before (null for the first of a run), and where the outcome goes.
+struct StepGate {
+    const double *parts;
+    int nparts;
+    double nmask;
+    const unsigned *err;
+    const StepLog *prev;
+    StepLog *log;
+};
 cudaError_t adam(float *theta, float *m, float *v, const float *grad, float lr, float b1, float b2, float eps,
-                 int step, cudaStream_t st);
+                 int step, const StepGate &gate, cudaStream_t st);
 cudaError_t pack(const float *theta, const Packed &p, cudaStream_t st);
 cudaError_t apply(const float *h, size_t pitch_in, const float *y, float kout, int nt, int np, float *out,
                   size_t pitch_out, cudaStream_t st);

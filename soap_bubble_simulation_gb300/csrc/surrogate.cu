@@ -65,6 +65,8 @@ struct Traj {
     uint32_t pairs = 0;
 };
 
+constexpr uint32_t kTrainRun = 4;  // training steps enqueued before their outcomes are read
+
 uint64_t splitmix64(uint64_t &x) {
     uint64_t z = (x += 0x9E3779B97F4A7C15ull);
     z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
@@ -102,6 +104,7 @@ struct sbs_surrogate {
     double *loss_part = nullptr;
     size_t loss_cap = 0;
     unsigned *err2 = nullptr;
+    sbs::nn::StepLog *log = nullptr;  // behind err2: the outcomes of a run of training steps
     float *scratch = nullptr;  // rollout check output
     size_t scratch_cap = 0;
     // training data
@@ -251,8 +254,10 @@ int layered_forward(sbs_surrogate *s, const Fields &fs, int nf, const GridDev &g
     return SBS_OK;
 }
 
-// loss (masked MSE against s->tgt) and the full gradient into s->grad
-int loss_and_grad(sbs_surrogate *s, const Fields &fs, int nf, const GridDev &g, double *loss) {
+// Enqueues the loss (masked MSE against s->tgt: *nlb partial sums in s->loss_part, to be divided by
+// *nmask) and the full gradient into s->grad.
+int enqueue_loss_and_grad(sbs_surrogate *s, const Fields &fs, int nf, const GridDev &g, int *loss_blocks,
+                          double *masked) {
     const int nt = g.nt, np = g.np;
     int rc = layered_forward(s, fs, nf, g);
     if (rc) return rc;
@@ -270,6 +275,17 @@ int loss_and_grad(sbs_surrogate *s, const Fields &fs, int nf, const GridDev &g, 
     SBS_CUDA_TRY(conv_backward_data(2, s->g2, s->pk, s->y1, s->g1, nf, nt, np, s->stream));
     SBS_CUDA_TRY(conv_backward_weight(1, s->g1, s->x0, s->partial, s->nblocks, s->grad, s->pk.err, nf, nt, np,
                                       s->stream));
+    *loss_blocks = nlb;
+    *masked = nmask;
+    return SBS_OK;
+}
+
+// The loss and the gradient, computed when the call returns.
+int loss_and_grad(sbs_surrogate *s, const Fields &fs, int nf, const GridDev &g, double *loss) {
+    int nlb = 0;
+    double nmask = 1.0;
+    int rc = enqueue_loss_and_grad(s, fs, nf, g, &nlb, &nmask);
+    if (rc) return rc;
     if (loss) {
         std::vector<double> lp(nlb);
         unsigned herr = 0;
@@ -378,8 +394,10 @@ int sbs_surrogate_create(uint64_t seed, sbs_surrogate **out) {
     s->pk.w4 = (float *)(s->pk.wb3 + 32 * 288);
     s->pk.b = s->pk.w4 + 288;
     s->partial = (float *)(pm + (pkb + 255) / 256 * 256);
-    if (cudaMalloc(&s->err2, 16) != cudaSuccess || cudaMemset(s->err2, 0, 16) != cudaSuccess)
+    if (cudaMalloc(&s->err2, 16 + sizeof(StepLog) * kTrainRun) != cudaSuccess ||
+        cudaMemset(s->err2, 0, 16) != cudaSuccess)
         return fail(set_error(SBS_E_NOMEM, "surrogate allocation failed"));
+    s->log = reinterpret_cast<StepLog *>(s->err2 + 4);
     s->pk.err = s->err2 + 2;  // words 0-1: masked_error's result
     // He-normal weights (fan-in 9 * ci), zero biases; the output layer starts small.
     std::vector<float> th(SBS_NN_PARAMS, 0.f);
@@ -645,6 +663,12 @@ int sbs_surrogate_train(sbs_surrogate *s, uint32_t n_train, uint32_t iters, uint
     for (uint32_t k = 0; k < n_train; ++k)
         for (uint32_t q = 0; q < s->data[k].pairs; ++q) pool.emplace_back(k, q);
     uint64_t st = seed;
+    // The outcomes of up to kTrainRun steps are read together. Reading each step's loss before its
+    // update left the GPU idle for 20 us a step; the update itself now decides (adam_kernel), and a step
+    // that fails leaves the parameters as they were before it, whatever was enqueued behind it.
+    StepLog log[kTrainRun];
+    const int adam0 = s->adam_step;
+    uint32_t first = 0;  // the first step whose outcome is not read yet
     for (uint32_t it = 0; it < iters; ++it) {
         Fields fs{};
         const float *h0[kMaxFields], *h1[kMaxFields];
@@ -659,17 +683,31 @@ int sbs_surrogate_train(sbs_surrogate *s, uint32_t n_train, uint32_t iters, uint
             kout[b] = t.fc.kout;
         }
         SBS_CUDA_TRY(targets(h0, h1, kout, (int)batch, nt, np, s->tgt, s->stream));
-        double loss = 0.0;
-        if ((rc = loss_and_grad(s, fs, (int)batch, *g, &loss))) return rc;
-        if (!std::isfinite(loss)) return set_error(SBS_E_NONFINITE, "training loss became non-finite at step %u", it);
-        if (losses) losses[it] = (float)loss;
+        const uint32_t at = it - first;
+        StepGate gate{};
+        if ((rc = enqueue_loss_and_grad(s, fs, (int)batch, *g, &gate.nparts, &gate.nmask))) return rc;
+        gate.parts = s->loss_part;
+        gate.err = s->pk.err;
+        gate.prev = at ? s->log + (at - 1) : nullptr;
+        gate.log = s->log + at;
         const double frac = iters > 1 ? (double)it / (double)(iters - 1) : 0.0;
         const float lr_t = (float)(lr * (0.05 + 0.95 * 0.5 * (1.0 + std::cos(M_PI * frac))));
         ++s->adam_step;
-        SBS_CUDA_TRY(adam(s->theta, s->m, s->v, s->grad, lr_t, 0.9f, 0.999f, 1e-8f, s->adam_step, s->stream));
+        SBS_CUDA_TRY(adam(s->theta, s->m, s->v, s->grad, lr_t, 0.9f, 0.999f, 1e-8f, s->adam_step, gate, s->stream));
         if ((rc = repack(s))) return rc;
+        if (at + 1 < kTrainRun && it + 1 < iters) continue;
+        SBS_CUDA_TRY(cudaMemcpyAsync(log, s->log, sizeof(StepLog) * (at + 1), cudaMemcpyDeviceToHost, s->stream));
+        SBS_CUDA_TRY(cudaStreamSynchronize(s->stream));
+        for (uint32_t k = 0; k <= at; ++k) {
+            if (log[k].code) {
+                s->adam_step = adam0 + (int)(first + k);
+                if (log[k].code == 2u) return tc_result(s, 2u);
+                return set_error(SBS_E_NONFINITE, "training loss became non-finite at step %u", first + k);
+            }
+            if (losses) losses[first + k] = (float)log[k].loss;
+        }
+        first = it + 1;
     }
-    SBS_CUDA_TRY(cudaStreamSynchronize(s->stream));
     return SBS_OK;
 }
 

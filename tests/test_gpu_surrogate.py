@@ -126,6 +126,50 @@ def test_layer4_strips_match_oracle(sbs, orc, net, nt, np_, nf):
         assert e <= 3e-2, (name, e)
 
 
+def first_draw(trajectory, n_train, batch, seed):
+    """The first step of a training run whose batch holds the trajectory (one pair each)."""
+    m, x = (1 << 64) - 1, seed
+    for it in range(1000):
+        for _ in range(batch):
+            x = (x + 0x9E3779B97F4A7C15) & m
+            z = ((x ^ (x >> 30)) * 0xBF58476D1CE4E5B9) & m
+            z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & m
+            if (z ^ (z >> 31)) % n_train == trajectory:
+                return it
+
+
+# Outcomes are read in runs of four steps; the failing step is the first, the second and the last of
+# a run, and one of a later run.
+@pytest.mark.parametrize("want", [0, 1, 3, 6])
+def test_non_finite_step_changes_nothing(sbs, want):
+    """A step whose loss is not finite is reported by its number, and neither it nor what was enqueued
+    behind it touches the parameters: they are those of a run that only had the steps before it."""
+    from soap_bubble_simulation_gb300 import synthetic as S
+
+    n_train, batch, nt, np_ = 5, 1, 24, 48
+    seed = next(q for q in range(1000) if first_draw(2, n_train, batch, q) == want)
+    nets = []
+    for nan in (True, False):
+        s = sbs.DrainageSurrogate(seed=3)
+        for k in range(n_train):
+            h = S.smooth_modes(nt, np_, seed=k).astype(np.float32)
+            if nan and k == 2:
+                h[nt // 2, 5] = np.nan
+            s.add_trajectory(h, S.surfactant_noise(nt, np_, seed=k), sbs.field_params(nt, np_), pairs=1)
+        nets.append(s)
+    start = nets[0].params
+    with pytest.raises(sbs.SbsError, match=f"step {want}$") as e:
+        nets[0].train(n_train, 40, batch=batch, lr=1e-30, seed=seed)
+    assert e.value.code == sbs._native.SBS_E_NONFINITE
+    assert np.abs(nets[0].params - start).max() <= 1e-28  # steps of this length move no weight
+    # the moments too: from here both nets go the same way, with the bad trajectory out of reach
+    if want:
+        nets[1].train(n_train, want, batch=batch, lr=1e-30, seed=seed)
+    good = [n.train(2, 3, batch=2, lr=1e-3, seed=9) for n in nets]
+    np.testing.assert_array_equal(good[0], good[1])
+    np.testing.assert_array_equal(nets[0].params, nets[1].params)
+
+
 def trained_surrogate(sbs, ntraj=24, nt=48, np_=96, iters=300, activation="gelu"):
     s = sbs.DrainageSurrogate(seed=3, activation=activation)
     g = np.random.default_rng(0)
