@@ -626,7 +626,7 @@ cudaError_t launch_wgrad(const TcWgradArgs &w, int nblocks, cudaStream_t st) {
 
 }  // namespace
 
-cudaError_t wgrad_tc(int cin, const bf16 *g, const bf16 *x, float *partial, int nblocks, unsigned *err, int nf, int nt,
+cudaError_t wgrad_tc(int cin, const bf16 *g, const bf16 *x, float *partial, int *nblocks, unsigned *err, int nf, int nt,
                      int np, cudaStream_t st) {
     TcWgradArgs w{};
     const int rows = nf * nt;
@@ -640,10 +640,13 @@ cudaError_t wgrad_tc(int cin, const bf16 *g, const bf16 *x, float *partial, int 
     w.np = np;
     w.cps = (np + kWgCells - 1) / kWgCells;
     w.nchunks = rows * w.cps;
+    // no block without a chunk: its partial row would be zeros that are written and added (64 x 128
+    // has 128 chunks for 304 blocks, rows of 37 KB)
+    *nblocks = std::min(*nblocks, w.nchunks);
     const WaitConfig wc = wait_config();
     w.wait_cycles = wc.cycles;
     w.stall = (wc.stall & SBS_STALL_TENSOR_COMMITS) ? 1 : 0;
-    return cin == 16 ? launch_wgrad<16>(w, nblocks, st) : launch_wgrad<32>(w, nblocks, st);
+    return cin == 16 ? launch_wgrad<16>(w, *nblocks, st) : launch_wgrad<32>(w, *nblocks, st);
 }
 
 cudaError_t conv_forward(int layer, const bf16 *in, const Packed &p, float *y, bf16 *a, int nf, int nt, int np,

@@ -571,7 +571,7 @@ cudaError_t conv_backward_weight(int layer, const bf16 *g, const bf16 *x, float 
     const int ci = layer == 1 ? 16 : 32;
     const int ow = layer == 1 ? SBS_NN_W1 : (layer == 2 ? SBS_NN_W2 : SBS_NN_W3);
     const int ob = layer == 1 ? SBS_NN_B1 : (layer == 2 ? SBS_NN_B2 : SBS_NN_B3);
-    cudaError_t e = wgrad_tc(ci, g, x, partial, nblocks, err, nf, nt, np, st);
+    cudaError_t e = wgrad_tc(ci, g, x, partial, &nblocks, err, nf, nt, np, st);
     if (e != cudaSuccess) return e;
     const int ncol = 32 * 9 * ci + 32;
     reduce_partials_kernel<<<(ncol + kRedCols - 1) / kRedCols, kRedCols * kRedRows, 0, st>>>(partial, nblocks, ci, 32,
