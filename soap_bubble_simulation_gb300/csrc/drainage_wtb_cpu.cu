@@ -88,7 +88,7 @@ struct Ctx {
     const double *vol_w;
     unsigned colbits[kMaxK]; // per step: 4 bits per front, the lane's columns inside it
     const TfeStep *tfe;      // the K steps' front records in shared memory
-    bool fronts;             // some step of the launch has a front
+    bool fronts;             // some cell of the warp's window lies inside a front of some step
     float4 *ring;            // this lane's row slots: ring[(slot * 2 + word) * 32]
 };
 
@@ -117,24 +117,37 @@ __device__ __forceinline__ void st_word(unsigned long long *p, unsigned tag, uns
 constexpr unsigned kWideTag = 0x80000000u;  // the slot holds a 256-bit partial (nine words), not 128 bits (four)
 constexpr unsigned kTagMask = 0x7fffffffu;
 
-// The payload of word p once it carries `tag`; *tagbits gets the whole tag. Gives up (and records
-// it) after the wait limit, or when another wait of the launch gave up.
-__device__ __forceinline__ unsigned wait_word(const unsigned long long *p, unsigned tag, unsigned *tagbits,
-                                              const RingX &x) {
-    unsigned long long v = ld_word(p);
-    if (((unsigned)(v >> 32) & kTagMask) != tag) {
-        const long long t0 = clock64();
-        for (unsigned tries = 1; ((unsigned)((v = ld_word(p)) >> 32) & kTagMask) != tag; ++tries) {
-            if (clock64() - t0 > x.limit || (tries % 64 == 0 && *(volatile unsigned *)x.status != 0u)) {
-                atomicOr(x.status, 1u);
-                *(volatile unsigned *)x.status_host = 1u;
-                *tagbits = tag;
-                return 0u;
-            }
+// The payloads of N adjacent words once all carry `tag`; *tagbits gets the last one's whole tag. The
+// words are read together: one trip to L2 (~700 cycles) where a wait for each in turn was five trips
+// for a narrow partial and ten for a wide one, at every level. Gives up (and records it) after the
+// wait limit, or when another wait of the launch gave up.
+template <int N>
+__device__ __forceinline__ void wait_words(const unsigned long long *p, unsigned tag, unsigned *w, unsigned *tagbits,
+                                           const RingX &x) {
+    long long t0 = 0;
+    for (unsigned tries = 0;; ++tries) {
+        unsigned long long v[N];
+        bool there = true;
+#pragma unroll
+        for (int k = 0; k < N; ++k) v[k] = ld_word(p + k);
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            there = there && ((unsigned)(v[k] >> 32) & kTagMask) == tag;
+            w[k] = (unsigned)v[k];
+        }
+        *tagbits = (unsigned)(v[N - 1] >> 32);
+        if (there) return;
+        if (tries == 0) {
+            t0 = clock64();
+        } else if (clock64() - t0 > x.limit || (tries % 64 == 0 && *(volatile unsigned *)x.status != 0u)) {
+            atomicOr(x.status, 1u);
+            *(volatile unsigned *)x.status_host = 1u;
+            *tagbits = tag;
+#pragma unroll
+            for (int k = 0; k < N; ++k) w[k] = 0u;
+            return;
         }
     }
-    *tagbits = (unsigned)(v >> 32);
-    return (unsigned)v;
 }
 
 // Exact sum of the lane's cells v (nv of them its own; hi and lo words in X2) over the block, and what
@@ -208,14 +221,11 @@ __device__ __forceinline__ float2 ring_gather(const RingX &x, RingShared &s, dou
         for (unsigned j = lane; j < x.narrive; j += 32) {
             const unsigned long long *p = x.slots + ((size_t)slot * x.nslots + j) * kRingWords;
             unsigned w[9], bits;
-            (void)wait_word(p + 3, tag, &bits, x);  // the last one written; the others are there or about to be
-#pragma unroll
-            for (int k = 0; k < 4; ++k) w[k] = wait_word(p + k, tag, &bits, x);
+            wait_words<4>(p, tag, w, &bits, x);
             fix128_add_words(a, w[0], w[1], w[2], w[3]);
             if (bits & kWideTag) {
                 mine = true;
-#pragma unroll
-                for (int k = 4; k < 9; ++k) w[k] = wait_word(p + k, tag, &bits, x);
+                wait_words<5>(p + 4, tag, w + 4, &bits, x);
                 fix_add(f, FixSum{((unsigned long long)w[1] << 32) | w[0], ((unsigned long long)w[3] << 32) | w[2],
                                   ((unsigned long long)w[5] << 32) | w[4], ((unsigned long long)w[7] << 32) | w[6],
                                   w[8], 0u});
@@ -238,10 +248,12 @@ __device__ __forceinline__ float2 ring_gather(const RingX &x, RingShared &s, dou
     return s.mean;
 }
 
-// Thins the cells of one row of step l that lie inside a front of that step (drainage.rs:425-460).
-template <bool X2, bool RAG>
+// Thins the cells of one row of step l that lie inside a front of that step (drainage.rs:425-460). In the
+// pipeline the product is formed for all cells and selected: a branch there would keep the levels'
+// chains of an iteration from overlapping.
+template <bool X2, bool SKIP, bool RAG>
 __device__ __forceinline__ void apply_fronts(const Ctx<RAG> &w, int l, int i, Row4 &oh, Row4 &ol) {
-    if (!w.fronts) return;
+    if (SKIP && !w.fronts) return;
     unsigned x = w.colbits[0];  // step l's, by selection: an index would move the context to local memory
 #pragma unroll
     for (int k = 1; k < kMaxK; ++k) x = l == k + 1 ? w.colbits[k] : x;
@@ -250,7 +262,7 @@ __device__ __forceinline__ void apply_fronts(const Ctx<RAG> &w, int l, int i, Ro
     x |= x >> 8;
     x |= x >> 4;
     x &= 0xfu;
-    if (!x) return;
+    if (SKIP && !x) return;
     const float2 fh = f2(w.tfe[l - 1].factor), fl = f2(w.tfe[l - 1].factor_lo);
     auto thin = [&](float2 &h, float2 &lo, bool first, bool second) {
         if (X2) {
@@ -318,7 +330,7 @@ __device__ __forceinline__ void iter(const Ctx<RAG> &w, int t, Row4 (&wh)[K][3],
             cpu_row<X2>(hc, wh[l - 1][UP], wh[l - 1][P], hlft, hrgt, lc, X2 ? wl[l - 1][UP] : zero,
                         X2 ? wl[l - 1][P] : zero, llft, lrgt, w.sco[i - w.t0], w.b, w.DR2, w.dt, w.crit,
                         oh, ol);
-            if (FRONTS) apply_fronts<X2>(w, l, i, oh, ol);
+            if (FRONTS) apply_fronts<X2, false>(w, l, i, oh, ol);
         }
         if (l < K) {
             wh[l][P] = oh;
@@ -359,6 +371,24 @@ __device__ __forceinline__ void interior_strip(const Ctx<RAG> &w, double &vacc) 
     const int t0 = w.t0, t1 = w.t0 + w.span;
 #pragma unroll
     for (int j = 0; j < kDepth; ++j) request_row<X2>(w, t0 + j);
+    if (FRONTS) {
+        // one copy of the iteration, its rows moved down after it: what bounds a launch with fronts is
+        // the fetch of its code (ncu at 1024 x 2048: 60 % of the warps' time), as the warps of an SM are
+        // in this loop and in the one without fronts at once
+#pragma unroll 1
+        for (int t = t0; t < t1; ++t) {
+            iter<K, 2, X2, VOL, FRONTS>(w, t, wh, wl, vacc);
+#pragma unroll
+            for (int l = 0; l < K; ++l)
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    wh[l][s] = wh[l][s + 1];
+                    wl[l][s] = wl[l][s + 1];
+                }
+        }
+        cp_async_wait<0>();
+        return;
+    }
     for (int t = t0; t < t1; t += 3) {
         iter<K, 0, X2, VOL, FRONTS>(w, t, wh, wl, vacc);
         if (t + 1 < t1) iter<K, 1, X2, VOL, FRONTS>(w, t + 1, wh, wl, vacc);
@@ -400,7 +430,7 @@ __device__ __forceinline__ void polar_strip(const Ctx<RAG> &w, Row4 *state, cons
             cpu_row<X2>(hc, hp, hn, hl, hr, lc, lp, ln, ll, lr, w.sco[at], w.b, w.DR2, w.dt, w.crit, oh, ol);
             // the pole's mean is of the stencil's values, before the fronts
             if (r == 1) ring_publish<X2>(oh, ol, nv, x, s, np, inv_np, slot);
-            if (FRONTS) apply_fronts<X2>(w, lev, row(r), oh, ol);
+            if (FRONTS) apply_fronts<X2, true>(w, lev, row(r), oh, ol);
             cell(r, 0) = oh;
             if (X2) cell(r, 1) = ol;
             hp = hc;
@@ -498,6 +528,7 @@ __global__ void __maxnreg__(kMaxRegs) wtbc_kernel(const StepArgs a) {
                 if (r >= s_tfe[l].fr[f].x && r <= s_tfe[l].fr[f].y) sel |= 0xfu << (4 * f);
             fsel[i] = sel;
         }
+        bool inside = false;  // one of the lane's cells
 #pragma unroll
         for (int l = 0; l < kMaxK; ++l) {
             unsigned bits = 0;
@@ -513,10 +544,11 @@ __global__ void __maxnreg__(kMaxRegs) wtbc_kernel(const StepArgs a) {
                     if (d < 0) d += np;
                     if (d < fr.w) bits |= 1u << (4 * f + k);
                 }
+                inside = inside || (bits >> (4 * f) != 0u && fr.x < w.t0 + w.span && fr.y >= w.t0);
             }
             w.colbits[l] = bits;
-            w.fronts = w.fronts || s_tfe[l].nf > 0;
         }
+        w.fronts = __any_sync(kFull, inside);
         __syncthreads();
     }
 
@@ -524,8 +556,12 @@ __global__ void __maxnreg__(kMaxRegs) wtbc_kernel(const StepArgs a) {
     if (polar)
         polar_strip<K, X2, VOL, FRONTS>(w, reinterpret_cast<Row4 *>(s_dyn) + threadIdx.x, s_x, s_ring, bottom,
                                         (double)np, a.inv_np, vacc);
-    else
-        interior_strip<K, X2, VOL, FRONTS>(w, vacc);
+    else if (FRONTS && w.fronts)
+        interior_strip<K, X2, VOL, true>(w, vacc);
+    else  // a front is narrow and starts at the equator: most windows of a launch with fronts meet none.
+          // 2000 steps with fronts, us per step with one unrolled loop for all and now: 2048 x 4096 20.9
+          // and 18.5 (plain f32 10.9 and 9.3), 1024 x 2048 11.0 and 7.6
+        interior_strip<K, X2, VOL, false>(w, vacc);
 
     if (VOL) {
         const double s = block_sum(vacc, s_vred);
