@@ -429,7 +429,7 @@ int sbs_foam_stream(const sbs_foam *f, void **out);
  * wavelengths) at nl <= 128 wavelengths wl_nm, contracted with the nl x 3
  * matrix cmf: rgb[3k+c] = sum_l R_l(k) cmf[3l+c]. The generalisation of the
  * reference's 7-sample CIE sum to a dense spectral contraction. Synchronous
- * in both memory modes (it reads back a device status flag). */
+ * in both memory modes (it waits for the kernel and its timeout word). */
 int sbs_spectral_rgb(const float *t_nm, const float *cos_i, const float *n_film, size_t n, const float *wl_nm,
                      uint32_t nl, const float *cmf, int mode, float *rgb, int mem, void *stream);
 
