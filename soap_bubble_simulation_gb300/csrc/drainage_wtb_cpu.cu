@@ -358,7 +358,7 @@ __host__ __device__ inline void strip_rows(int by, int ns, int nt, int K, int &r
 }
 
 // The pipeline over a whole interior strip: its rows are neither poles nor next to one at any level.
-template <int K, bool X2, bool VOL, bool FRONTS, bool RAG>
+template <int K, bool X2, bool VOL, bool FRONTS, bool ROLL, bool RAG>
 __device__ __forceinline__ void interior_strip(const Ctx<RAG> &w, double &vacc) {
     Row4 wh[K][3], wl[K][3];
 #pragma unroll
@@ -371,7 +371,7 @@ __device__ __forceinline__ void interior_strip(const Ctx<RAG> &w, double &vacc) 
     const int t0 = w.t0, t1 = w.t0 + w.span;
 #pragma unroll
     for (int j = 0; j < kDepth; ++j) request_row<X2>(w, t0 + j);
-    if (FRONTS) {
+    if (ROLL) {
         // one copy of the iteration, its rows moved down after it: what bounds a launch with fronts is
         // the fetch of its code (ncu at 1024 x 2048: 60 % of the warps' time), as the warps of an SM are
         // in this loop and in the one without fronts at once
@@ -386,13 +386,12 @@ __device__ __forceinline__ void interior_strip(const Ctx<RAG> &w, double &vacc) 
                     wl[l][s] = wl[l][s + 1];
                 }
         }
-        cp_async_wait<0>();
-        return;
-    }
-    for (int t = t0; t < t1; t += 3) {
-        iter<K, 0, X2, VOL, FRONTS>(w, t, wh, wl, vacc);
-        if (t + 1 < t1) iter<K, 1, X2, VOL, FRONTS>(w, t + 1, wh, wl, vacc);
-        if (t + 2 < t1) iter<K, 2, X2, VOL, FRONTS>(w, t + 2, wh, wl, vacc);
+    } else {
+        for (int t = t0; t < t1; t += 3) {
+            iter<K, 0, X2, VOL, FRONTS>(w, t, wh, wl, vacc);
+            if (t + 1 < t1) iter<K, 1, X2, VOL, FRONTS>(w, t + 1, wh, wl, vacc);
+            if (t + 2 < t1) iter<K, 2, X2, VOL, FRONTS>(w, t + 2, wh, wl, vacc);
+        }
     }
     cp_async_wait<0>();  // every copy was consumed; nothing may still be landing at exit
 }
@@ -557,11 +556,12 @@ __global__ void __maxnreg__(kMaxRegs) wtbc_kernel(const StepArgs a) {
         polar_strip<K, X2, VOL, FRONTS>(w, reinterpret_cast<Row4 *>(s_dyn) + threadIdx.x, s_x, s_ring, bottom,
                                         (double)np, a.inv_np, vacc);
     else if (FRONTS && w.fronts)
-        interior_strip<K, X2, VOL, true>(w, vacc);
+        interior_strip<K, X2, VOL, true, true>(w, vacc);
     else  // a front is narrow and starts at the equator: most windows of a launch with fronts meet none.
-          // 2000 steps with fronts, us per step with one unrolled loop for all and now: 2048 x 4096 20.9
-          // and 18.5 (plain f32 10.9 and 9.3), 1024 x 2048 11.0 and 7.6
-        interior_strip<K, X2, VOL, false>(w, vacc);
+          // Steps with fronts, us each over 4000 late ones, with one unrolled loop for all, with this one
+          // unrolled, rolled: 2048 x 4096 22.7, 19.7, 18.7 (plain f32 11.6, 9.8, 10.0: it stays unrolled);
+          // 1024 x 2048 14.7, 9.0, 7.8 (plain f32 6.5, 4.5, 4.4)
+        interior_strip<K, X2, VOL, false, FRONTS && X2>(w, vacc);
 
     if (VOL) {
         const double s = block_sum(vacc, s_vred);
