@@ -18,7 +18,8 @@
 // spatial hash of cells (edge half of 6 r_max + skin, so the 5 x 5 x 5 cells around a bubble hold
 // all its candidates), counts each bubble's candidates (a warp per bubble), orders the bubbles by
 // descending count, collects the candidates again into each bubble's column and sorts each column
-// by index with a warp-wide bitonic sort in registers. The lists of 32 bubbles at consecutive
+// by index with a warp-wide bitonic sort in registers (a block-wide one beyond 2048 entries: under the
+// default physics a cluster contracts to lists of that length and more). The lists of 32 bubbles at consecutive
 // positions of that order are interleaved (entry t of the bubble at position q at
 // goff[q / 32] + 32 t + q % 32): the force pass reads them coalesced and, the lengths of
 // neighbouring positions being nearly equal, its lanes idle little.
@@ -48,14 +49,15 @@ namespace {
 
 constexpr float kPi = 3.14159265358979323846f;
 constexpr float kMaxSpeed = 0.1f;   // foam_dynamics.rs:194
-constexpr int kMaxCand = 2048;      // neighbour-list entries per bubble (the shared-memory sort buffer)
+constexpr int kListBins = 2048;     // list lengths told apart by the order of the bubbles; longer ones share a bin
+constexpr int kWarpSort = 2048;     // entries of a list that one warp sorts in its share of shared memory
 constexpr int kThreads = 256;
 constexpr uint32_t kNone = 0xffffffffu;
 constexpr unsigned long long kNoPair = ~0ull;
 
 // kFaultWalk: a bubble's candidate walk collected a different number of entries than its count
 // pass (the two passes make the same decisions, so this means a fault of the build itself).
-enum Fault : uint32_t { kFaultNone = 0, kFaultCapacity = 1, kFaultDense = 2, kFaultWalk = 3 };
+enum Fault : uint32_t { kFaultNone = 0, kFaultCapacity = 1, kFaultWalk = 3 };
 
 // Device-side control block.
 struct Ctl {
@@ -69,7 +71,9 @@ struct Ctl {
     unsigned long long coal_key;  // first connection (i << 32 | j) whose Weber number is over the threshold
     uint32_t merged_a, merged_b;  // ids merged by the last step, kNone if none
     float inv_cell, skin, cell, rmax;
-    uint32_t list_total, dense_bubble, dense_count, pad1;
+    unsigned long long list_total;  // entries that the lists need
+    uint32_t long_lists;            // some list is longer than kWarpSort
+    uint32_t pad1;
 };
 
 struct Phys {
@@ -214,7 +218,7 @@ struct ListArgs {
     uint32_t *split;        // entries j < k of each list (the sorted list's lower part)
     uint32_t *perm;         // bubbles by descending list length: the order of the 32-bubble groups
     uint32_t *inv;          // position of each bubble in perm
-    uint32_t *mhist, *mstart;  // bubbles per list length (kMaxCand + 1 bins, longest first)
+    uint32_t *mhist, *mstart;  // bubbles per list length (kListBins + 1 bins, longest first)
     uint32_t *gcap;         // largest list length of each 32-bubble group
     uint32_t *goff;         // group offsets (ngroups + 1)
     uint32_t *nbr;          // interleaved lists
@@ -251,6 +255,8 @@ __global__ void __launch_bounds__(1024) list_begin_kernel(ListArgs a, int forced
             c->rmax = m;
             c->skin = skin;
             c->stale = kNone;
+            c->list_total = 0;
+            c->long_lists = 0;
             c->go = 1;
         }
     }
@@ -325,8 +331,7 @@ __global__ void __launch_bounds__(1024) scan_kernel(const uint32_t *in, uint32_t
     if (threadIdx.x == 0) {
         out[count] = s_carry;
         if (mode == 1) {
-            c->list_total = s_carry;
-            if (s_carry > a.nbr_cap) c->fault = kFaultCapacity;
+            if (c->list_total > a.nbr_cap) c->fault = kFaultCapacity;  // the offsets may have wrapped then
         }
     }
 }
@@ -482,16 +487,13 @@ __global__ void __launch_bounds__(kListWarps * 32) list_count_kernel(ListArgs a)
              [&](uint32_t, bool ok) { m += __popc(__ballot_sync(0xffffffffu, ok)); });
         if (lane == 0) {
             a.cnt[k] = m;
-            atomicAdd(a.mhist + (kMaxCand - min(m, (uint32_t)kMaxCand)), 1u);
-            if (m > (uint32_t)kMaxCand && atomicCAS(&c->fault, kFaultNone, kFaultDense) == kFaultNone) {
-                c->dense_bubble = k;
-                c->dense_count = m;
-            }
+            atomicAdd(a.mhist + (kListBins - min(m, (uint32_t)kListBins)), 1u);
+            if (m > (uint32_t)kWarpSort) atomicOr(&c->long_lists, 1u);
         }
     }
 }
 
-// Lists longer than 1024 (rare): bitonic sort in shared memory.
+// Lists of 1025 to kWarpSort entries (rare): bitonic sort in shared memory.
 __device__ __noinline__ uint32_t sort_smem(uint32_t *buf, uint32_t m, uint32_t k, uint32_t *col, int lane) {
     uint32_t P = 1;
     while (P < m) P <<= 1;
@@ -527,20 +529,24 @@ __global__ void list_order_kernel(ListArgs a) {
     if (!c->go || c->fault != kFaultNone) return;
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= c->n[a.npar]) return;
-    const uint32_t pos = atomicAdd(a.mstart + (kMaxCand - a.cnt[k]), 1u);
+    const uint32_t pos = atomicAdd(a.mstart + (kListBins - min(a.cnt[k], (uint32_t)kListBins)), 1u);
     a.perm[pos] = k;
     a.inv[k] = pos;
 }
 
-// The largest list length of each group of 32 consecutive positions of the order.
+// The largest list length of each group of 32 consecutive positions of the order, and the entries of
+// all groups (in 64 bits: the offsets have 32).
 __global__ void list_gcap_kernel(ListArgs a) {
-    const Ctl *c = a.ctl;
+    Ctl *c = a.ctl;
     if (!c->go || c->fault != kFaultNone) return;
     const uint32_t n = c->n[a.npar];
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t m = t < n ? a.cnt[a.perm[t]] : 0u;
     for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && t < ((n + 31) & ~31u)) a.gcap[t >> 5] = m;
+    if ((threadIdx.x & 31) == 0 && t < ((n + 31) & ~31u)) {
+        a.gcap[t >> 5] = m;
+        atomicAdd(&c->list_total, ((m + 31u) & ~31u) * 32ull);
+    }
 }
 
 // A warp per bubble: collects the candidates again, in the walk's order, straight into the bubble's
@@ -594,10 +600,32 @@ __device__ __forceinline__ uint32_t sort_column(uint32_t *col, uint32_t m, uint3
     return below;
 }
 
+// Bitonic sort of m entries at v, `step` words apart, by the block. Every exchange moves the smaller
+// entry down (a merge begins with mirrored pairs), so the entries that a power of two would need
+// beyond m are larger than all and stay where they are.
+__device__ void block_sort(uint32_t *v, size_t step, uint32_t m) {
+    for (uint32_t size = 2; (size >> 1) < m; size <<= 1)
+        for (uint32_t half = size >> 1; half > 0; half >>= 1) {
+            const uint32_t flip = half == size >> 1 ? size - 1 : half;
+            for (uint32_t p = threadIdx.x;; p += blockDim.x) {
+                const uint32_t i = ((p & ~(half - 1)) << 1) | (p & (half - 1)), l = i ^ flip;
+                if (i >= m) break;
+                if (l >= m) continue;
+                const uint32_t x = v[i * step], y = v[l * step];
+                if (x > y) {
+                    v[i * step] = y;
+                    v[l * step] = x;
+                }
+            }
+            __syncthreads();
+        }
+}
+
 // A warp per bubble: sorts its column by index in registers (bitonic; in shared memory beyond 1024
-// entries) and records the length of its lower part.
+// entries) and records the length of its lower part. Lists longer than kWarpSort, of clusters that have
+// contracted, are the whole block's afterwards: in its shared memory, or in place.
 __global__ void __launch_bounds__(kListWarps * 32, 4) list_sort_kernel(ListArgs a) {
-    __shared__ uint32_t s_buf[kListWarps][kMaxCand];
+    __shared__ uint32_t s_buf[kListWarps][kWarpSort];
     const Ctl *c = a.ctl;
     if (!c->go || c->fault != kFaultNone) return;
     const uint32_t n = c->n[a.npar];
@@ -605,6 +633,7 @@ __global__ void __launch_bounds__(kListWarps * 32, 4) list_sort_kernel(ListArgs 
     uint32_t *buf = s_buf[threadIdx.x >> 5];
     for (uint32_t k = blockIdx.x * kListWarps + (threadIdx.x >> 5); k < n; k += gridDim.x * kListWarps) {
         const uint32_t m = a.cnt[k];
+        if (m > (uint32_t)kWarpSort) continue;
         const uint32_t pos = a.inv[k];
         uint32_t *col = a.nbr + a.goff[pos >> 5] + (pos & 31);
         uint32_t below;
@@ -622,6 +651,28 @@ __global__ void __launch_bounds__(kListWarps * 32, 4) list_sort_kernel(ListArgs 
         for (int o = 16; o; o >>= 1) below += __shfl_xor_sync(0xffffffffu, below, o);
         if (lane == 0) a.split[k] = below;
         __syncwarp();
+    }
+    if (!c->long_lists) return;
+    for (uint32_t r = 0;; ++r) {  // the block's bubbles again
+        const uint32_t k = (blockIdx.x + r / kListWarps * gridDim.x) * kListWarps + r % kListWarps;
+        if (k >= n) break;
+        const uint32_t m = a.cnt[k];
+        if (m <= (uint32_t)kWarpSort) continue;
+        const uint32_t pos = a.inv[k];
+        uint32_t *col = a.nbr + a.goff[pos >> 5] + (pos & 31);
+        const bool fits = m <= (uint32_t)(kListWarps * kWarpSort);
+        uint32_t *v = fits ? &s_buf[0][0] : col;
+        const size_t step = fits ? 1 : 32;
+        __syncthreads();  // the buffer is free
+        for (uint32_t t = threadIdx.x; fits && t < m; t += blockDim.x) v[t] = col[(size_t)t * 32];
+        __syncthreads();
+        block_sort(v, step, m);
+        for (uint32_t t = threadIdx.x; t < m; t += blockDim.x) {
+            const uint32_t x = v[t * step];
+            if (fits) col[(size_t)t * 32] = x;
+            if (x < k && (t + 1 == m || v[(t + 1) * step] > k)) a.split[k] = t + 1;  // k itself is not listed
+            if (t == 0 && x > k) a.split[k] = 0;
+        }
     }
 }
 
@@ -1111,13 +1162,13 @@ void enqueue_list(sbs_foam_sim *s, bool forced, float skin) {
     ListArgs a = list_args(s);
     s->list_skin = skin;
     cudaMemsetAsync(s->bcount, 0, sizeof(uint32_t) * (s->mask + 1), s->stream);
-    cudaMemsetAsync(s->mhist, 0, sizeof(uint32_t) * (kMaxCand + 1), s->stream);
+    cudaMemsetAsync(s->mhist, 0, sizeof(uint32_t) * (kListBins + 1), s->stream);
     list_begin_kernel<<<1, 1024, 0, s->stream>>>(a, forced ? 1 : 0, skin);
     list_bin_kernel<<<blocks(s->n_cap), kThreads, 0, s->stream>>>(a);
     scan_kernel<<<1, 1024, 0, s->stream>>>(s->bcount, s->bstart, s->mask + 1, 0, a);
     list_scatter_kernel<<<blocks(s->n_cap), kThreads, 0, s->stream>>>(a);
     list_count_kernel<<<s->list_blocks, kListWarps * 32, 0, s->stream>>>(a);
-    scan_kernel<<<1, 1024, 0, s->stream>>>(s->mhist, s->mstart, kMaxCand + 1, 0, a);
+    scan_kernel<<<1, 1024, 0, s->stream>>>(s->mhist, s->mstart, kListBins + 1, 0, a);
     list_order_kernel<<<blocks(s->n_cap), kThreads, 0, s->stream>>>(a);
     list_gcap_kernel<<<blocks(s->n_cap), kThreads, 0, s->stream>>>(a);
     scan_kernel<<<1, 1024, 0, s->stream>>>(s->gcap, s->goff, 0, 1, a);
@@ -1188,6 +1239,17 @@ int read_ctl(sbs_foam_sim *s, Ctl *h) {
     return SBS_OK;
 }
 
+// Larger storage for lists that need `total` entries and half as many again, at most what 32-bit offsets reach;
+// the list has to be built anew whatever comes of it.
+int grow_list(sbs_foam_sim *s, unsigned long long total) {
+    constexpr unsigned long long most = 0xfffffc00ull;
+    s->list_invalid = true;
+    SBS_CUDA_TRY(cudaMemsetAsync(&s->ctl->fault, 0, sizeof(uint32_t), s->stream));
+    if (total > most)
+        return set_error(SBS_E_INVALID, "foam too dense: %llu pairs within 3 (r_a + r_b) + skin (limit %llu)", total, most);
+    return alloc_list(s, (size_t)std::min(total + total / 2 + 1024, most));
+}
+
 // Builds the neighbour list for the current state, growing its storage as needed.
 int rebuild_now(sbs_foam_sim *s, float skin) {
     for (int attempt = 0; attempt < 3; ++attempt) {
@@ -1196,17 +1258,12 @@ int rebuild_now(sbs_foam_sim *s, float skin) {
         Ctl h;
         int rc = read_ctl(s, &h);
         if (rc) return rc;
-        if (h.fault == kFaultDense)
-            return set_error(SBS_E_INVALID,
-                             "foam too dense: bubble %u has %u neighbours within 3 (r_a + r_b) + skin (limit %d)",
-                             h.dense_bubble, h.dense_count, kMaxCand);
         if (h.fault == kFaultWalk) return set_error(SBS_E_STATE, "foam neighbour list: walk and count passes disagree");
         if (h.fault == kFaultNone) {
             s->list_invalid = false;
             return SBS_OK;
         }
-        SBS_CUDA_TRY(cudaMemsetAsync(&s->ctl->fault, 0, sizeof(uint32_t), s->stream));
-        if ((rc = alloc_list(s, (size_t)h.list_total + h.list_total / 2 + 1024))) return rc;
+        if ((rc = grow_list(s, h.list_total))) return rc;
     }
     return set_error(SBS_E_CUDA, "foam neighbour list: could not size the list");
 }
@@ -1323,8 +1380,8 @@ int sbs_foam_sim_create(uint32_t n, const float *position, const float *radius, 
     if (e == cudaSuccess) e = cudaMalloc(&s->split, sizeof(uint32_t) * n);
     if (e == cudaSuccess) e = cudaMalloc(&s->perm, sizeof(uint32_t) * n);
     if (e == cudaSuccess) e = cudaMalloc(&s->inv, sizeof(uint32_t) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&s->mhist, sizeof(uint32_t) * (kMaxCand + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&s->mstart, sizeof(uint32_t) * (kMaxCand + 2));
+    if (e == cudaSuccess) e = cudaMalloc(&s->mhist, sizeof(uint32_t) * (kListBins + 1));
+    if (e == cudaSuccess) e = cudaMalloc(&s->mstart, sizeof(uint32_t) * (kListBins + 2));
     if (e == cudaSuccess) e = cudaMalloc(&s->gcap, sizeof(uint32_t) * groups);
     if (e == cudaSuccess) e = cudaMalloc(&s->goff, sizeof(uint32_t) * (groups + 1));
     if (e != cudaSuccess) return fail(e);
@@ -1430,13 +1487,7 @@ int sbs_foam_sim_step(sbs_foam_sim *s, float dt, uint32_t steps) {
         }
         // The list outgrew its storage at a rebuild: the steps from there on did nothing. Grow it and
         // continue.
-        if (h.fault == kFaultDense)
-            return set_error(SBS_E_INVALID,
-                             "foam too dense: bubble %u has %u neighbours within 3 (r_a + r_b) + skin (limit %d)",
-                             h.dense_bubble, h.dense_count, kMaxCand);
-        SBS_CUDA_TRY(cudaMemsetAsync(&s->ctl->fault, 0, sizeof(uint32_t), s->stream));
-        if ((rc = alloc_list(s, (size_t)h.list_total + h.list_total / 2 + 1024))) return rc;
-        s->list_invalid = true;
+        if ((rc = grow_list(s, h.list_total))) return rc;
     }
     return SBS_OK;
 }

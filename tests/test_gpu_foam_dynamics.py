@@ -242,3 +242,40 @@ def test_runs_of_steps_match_oracle(fd, orc, dt, calls):
         _same_state(sim, want)
         np.testing.assert_array_equal(sim.compute_forces(), orc.foam_forces(sim.physics, want["position"], want["radius"],
                                                                             velocity=want["velocity"]))
+
+
+@pytest.mark.parametrize("n,lo,hi", [(2500, 0.03, 0.09), (3000, 0.3, 0.4), (8250, 0.5, 0.6)])
+def test_lists_of_any_length(fd, orc, n, lo, hi):
+    """Lists on both sides of what one warp sorts (2048), of nearly all bubbles, and of more than the
+    block's shared memory holds (8192): forces in the reference's order."""
+    pos, rad = fd.fcc_foam(n, min_radius=lo, max_radius=hi, seed=71)
+    d = np.linalg.norm(pos[:, None, :].astype(np.float32) - pos[None, : n // 8], axis=2)
+    longest = (d < 3.0 * (rad[:, None] + rad[None, : n // 8])).sum(0).max()
+    assert longest > (8192 if n > 8192 else 2048)
+    sim = fd.FoamSimulator(pos, rad)
+    idx = np.unique(np.concatenate([[0, 1, n - 2, n - 1], np.random.default_rng(72).integers(0, n, 40)]))
+    np.testing.assert_array_equal(sim.compute_forces()[idx], orc.foam_forces_subset(sim.physics, pos, rad, idx))
+    sim.step(1e-3, 2)
+    b = sim.bubbles()
+    np.testing.assert_array_equal(sim.compute_forces()[idx],
+                                  orc.foam_forces_subset(sim.physics, b["position"], b["radius"], idx,
+                                                         velocity=b["velocity"]))
+
+
+def test_contracting_cluster_goes_on(fd, orc):
+    """Under the default physics a cluster contracts until some bubbles have more than 2048 others in
+    range (8000 bubbles: after 3240 steps of 1 ms); it is stepped on."""
+    pos, rad = fd.fcc_foam(8000, seed=3)
+    sim = fd.FoamSimulator(pos, rad)
+    for _ in range(17):
+        sim.step(1e-3, 200)
+    b = sim.bubbles()
+    near = 0
+    for i in range(0, 8000, 250):
+        d = np.linalg.norm(b["position"][i : i + 250, None] - b["position"][None], axis=2)
+        near = max(near, int((d < 3.0 * (b["radius"][i : i + 250, None] + b["radius"][None]) + 0.02).sum(1).max()))
+    assert near > 2048
+    idx = np.arange(0, 8000, 333)
+    np.testing.assert_array_equal(sim.compute_forces()[idx],
+                                  orc.foam_forces_subset(sim.physics, b["position"], b["radius"], idx,
+                                                         velocity=b["velocity"]))
