@@ -1252,6 +1252,7 @@ int grow_list(sbs_foam_sim *s, unsigned long long total) {
 
 // Builds the neighbour list for the current state, growing its storage as needed.
 int rebuild_now(sbs_foam_sim *s, float skin) {
+    s->list_invalid = true;
     for (int attempt = 0; attempt < 3; ++attempt) {
         enqueue_list(s, true, skin);
         SBS_CUDA_TRY(cudaGetLastError());
@@ -1271,6 +1272,76 @@ int rebuild_now(sbs_foam_sim *s, float skin) {
 int current_n(sbs_foam_sim *s, uint32_t *n) {
     SBS_CUDA_TRY(cudaMemcpyAsync(n, &s->ctl->n[s->npar], sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
     SBS_CUDA_TRY(cudaStreamSynchronize(s->stream));
+    return SBS_OK;
+}
+
+// `steps` steps of the cluster, in runs.
+int run_cluster(sbs_foam_sim *s, float dt, uint32_t steps) {
+    const bool coal = s->phys.coalescence_enabled != 0;
+    const float skin = skin_for(s, dt);
+    if (skin != s->list_skin) s->list_invalid = true;  // a new dt: a list built for this step size
+    s->conn_cached = false;
+    uint32_t done = 0;
+    while (done < steps) {
+        int rc;
+        if (s->list_invalid) {
+            if ((rc = rebuild_now(s, skin))) return rc;
+        } else if (s->list_stale) {
+            enqueue_list(s, true, skin);
+        }
+        s->list_stale = false;
+        // The steps of a run are enqueued at once; they read the list's state on the device. A step
+        // after which the list no longer holds stops the run: the later ones do nothing, and the next
+        // run starts with a rebuild. Enqueued before every step instead, a rebuild that has nothing to
+        // do is 13 launches, 50 us where the forces of 40000 bubbles take 100; that pays only where
+        // every step needs one (it saves the wait at the end of the run).
+        const bool eager = s->quiet <= 1;
+        const uint32_t run = std::min(steps - done, eager ? kEagerRun : s->quiet);
+        const int cur0 = s->cur, npar0 = s->npar;
+        SBS_CUDA_TRY(cudaMemsetAsync(&s->ctl->steps_done, 0, sizeof(uint32_t), s->stream));
+        for (uint32_t k = 0; k < run; ++k) {
+            if (eager && k) enqueue_list(s, false, skin);
+            DynArgs a = dyn_args(s, dt, s->cur, s->cur ^ 1);
+            a.step = k + 1;
+            launch_forces(s, a);
+            if (coal || done + k + 1 == steps) connections_kernel<<<blocks(s->n_cap, 32), kThreads, 0, s->stream>>>(a);
+            if (coal) {
+                DynArgs m = dyn_args(s, dt, s->cur ^ 1, s->cur);
+                m.step = k + 1;
+                merge_kernel<<<blocks(s->n_cap), kThreads, 0, s->stream>>>(m);
+                s->npar ^= 1;
+            } else {
+                s->cur ^= 1;
+            }
+        }
+        SBS_CUDA_TRY(cudaGetLastError());
+        Ctl h;
+        if ((rc = read_ctl(s, &h))) return rc;
+        s->stepped = true;
+        // the buffer parities of the last completed step
+        done += h.steps_done;
+        if (coal) {
+            s->cur = cur0;
+            s->npar = npar0 ^ (int)(h.steps_done & 1);
+            s->conn_buf = cur0 ^ 1;
+            s->conn_npar = s->npar ^ 1;
+        } else {
+            s->cur = cur0 ^ (int)(h.steps_done & 1);
+            s->conn_buf = s->cur;
+            s->conn_npar = s->npar;
+        }
+        s->list_stale = h.stale != kNone;
+        if (h.fault == kFaultWalk) return set_error(SBS_E_STATE, "foam neighbour list: walk and count passes disagree");
+        if (h.fault == kFaultNone) {
+            if (eager) s->quiet = 2;  // see whether it is still so
+            else if (s->list_stale) s->quiet = std::min(2 * h.steps_done - (h.steps_done == 1), kLongestRun);
+            else if (run == s->quiet) s->quiet = std::min(2 * run, kLongestRun);
+            continue;
+        }
+        // The list outgrew its storage at a rebuild: the steps from there on did nothing. Grow it and
+        // continue.
+        if ((rc = grow_list(s, h.list_total))) return rc;
+    }
     return SBS_OK;
 }
 
@@ -1424,72 +1495,14 @@ int sbs_foam_sim_step(sbs_foam_sim *s, float dt, uint32_t steps) {
     SBS_CHECK_ARG(s != nullptr, "handle is null");
     SBS_CHECK_ARG(std::isfinite(dt), "dt must be finite");
     if (steps == 0) return SBS_OK;
-    const bool coal = s->phys.coalescence_enabled != 0;
-    const float skin = skin_for(s, dt);
-    if (skin != s->list_skin) s->list_invalid = true;  // a new dt: a list built for this step size
-    s->conn_cached = false;
-    uint32_t done = 0;
-    while (done < steps) {
-        int rc;
-        if (s->list_invalid) {
-            if ((rc = rebuild_now(s, skin))) return rc;
-        } else if (s->list_stale) {
-            enqueue_list(s, true, skin);
-        }
-        s->list_stale = false;
-        // The steps of a run are enqueued at once; they read the list's state on the device. A step
-        // after which the list no longer holds stops the run: the later ones do nothing, and the next
-        // run starts with a rebuild. Enqueued before every step instead, a rebuild that has nothing to
-        // do is 13 launches, 50 us where the forces of 40000 bubbles take 100; that pays only where
-        // every step needs one (it saves the wait at the end of the run).
-        const bool eager = s->quiet <= 1;
-        const uint32_t run = std::min(steps - done, eager ? kEagerRun : s->quiet);
-        const int cur0 = s->cur, npar0 = s->npar;
-        SBS_CUDA_TRY(cudaMemsetAsync(&s->ctl->steps_done, 0, sizeof(uint32_t), s->stream));
-        for (uint32_t k = 0; k < run; ++k) {
-            if (eager && k) enqueue_list(s, false, skin);
-            DynArgs a = dyn_args(s, dt, s->cur, s->cur ^ 1);
-            a.step = k + 1;
-            launch_forces(s, a);
-            if (coal || done + k + 1 == steps) connections_kernel<<<blocks(s->n_cap, 32), kThreads, 0, s->stream>>>(a);
-            if (coal) {
-                DynArgs m = dyn_args(s, dt, s->cur ^ 1, s->cur);
-                m.step = k + 1;
-                merge_kernel<<<blocks(s->n_cap), kThreads, 0, s->stream>>>(m);
-                s->npar ^= 1;
-            } else {
-                s->cur ^= 1;
-            }
-        }
-        SBS_CUDA_TRY(cudaGetLastError());
-        Ctl h;
-        if ((rc = read_ctl(s, &h))) return rc;
-        s->stepped = true;
-        if (h.fault == kFaultWalk) return set_error(SBS_E_STATE, "foam neighbour list: walk and count passes disagree");
-        // the buffer parities of the last completed step
-        done += h.steps_done;
-        if (coal) {
-            s->cur = cur0;
-            s->npar = npar0 ^ (int)(h.steps_done & 1);
-            s->conn_buf = cur0 ^ 1;
-            s->conn_npar = s->npar ^ 1;
-        } else {
-            s->cur = cur0 ^ (int)(h.steps_done & 1);
-            s->conn_buf = s->cur;
-            s->conn_npar = s->npar;
-        }
-        s->list_stale = h.stale != kNone;
-        if (h.fault == kFaultNone) {
-            if (eager) s->quiet = 2;  // see whether it is still so
-            else if (s->list_stale) s->quiet = std::min(2 * h.steps_done - (h.steps_done == 1), kLongestRun);
-            else if (run == s->quiet) s->quiet = std::min(2 * run, kLongestRun);
-            continue;
-        }
-        // The list outgrew its storage at a rebuild: the steps from there on did nothing. Grow it and
-        // continue.
-        if ((rc = grow_list(s, h.list_total))) return rc;
+    const int rc = run_cluster(s, dt, steps);
+    if (rc) {
+        // The list may be half built (new lengths, old storage or none), so nothing may read the last
+        // step's connections from it: queries start from the state and a list of their own.
+        s->list_invalid = true;
+        s->stepped = s->conn_cached = false;
     }
-    return SBS_OK;
+    return rc;
 }
 
 int sbs_foam_sim_counts(sbs_foam_sim *s, uint32_t *bubbles, uint32_t *connections) {

@@ -279,3 +279,25 @@ def test_contracting_cluster_goes_on(fd, orc):
     np.testing.assert_array_equal(sim.compute_forces()[idx],
                                   orc.foam_forces_subset(sim.physics, b["position"], b["radius"], idx,
                                                          velocity=b["velocity"]))
+
+
+def test_queries_after_a_failed_step(sbs, fd):
+    """A step whose lists cannot be built (a dt that puts every pair in range: more than 32-bit offsets
+    reach) leaves the cluster at the last step: connections, forces and further steps are a twin's."""
+    pos, rad = fd.fcc_foam(70000, seed=5)
+    sim, twin = fd.FoamSimulator(pos, rad), fd.FoamSimulator(pos, rad)
+    for s in (sim, twin):
+        s.step(1e-3, 2)
+    want = twin.connections()
+    with pytest.raises(sbs.SbsError, match="too dense"):
+        sim.step(100.0, 1)
+    assert sim.bubble_count() == twin.bubble_count()
+    np.testing.assert_array_equal(sim.compute_forces(), twin.compute_forces())
+    assert len(want) and sim.connection_count() == len(want)
+    got = sim.connections()
+    for k in want.dtype.names:
+        np.testing.assert_array_equal(got[k], want[k])
+    for s in (sim, twin):
+        s.step(1e-3, 3)
+    for k, v in sim.bubbles().items():
+        np.testing.assert_array_equal(v, twin.bubbles()[k])
