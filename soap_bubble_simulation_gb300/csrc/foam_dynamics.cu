@@ -1642,7 +1642,7 @@ int sbs_foam_sim_forces(sbs_foam_sim *s, float *forces, int mem) {
                 s->conn_cache.swap(keep);
                 s->conn_cached = true;
             }
-            enqueue_list(s, false, s->list_skin);
+            if ((rc = rebuild_now(s, s->list_skin))) return rc;  // grown where it has become too small
             s->list_stale = false;
         }
     }

@@ -301,3 +301,27 @@ def test_queries_after_a_failed_step(sbs, fd):
         s.step(1e-3, 3)
     for k, v in sim.bubbles().items():
         np.testing.assert_array_equal(v, twin.bubbles()[k])
+
+
+def test_forces_where_the_list_outgrows_its_storage(fd, orc):
+    """Bubbles on a shrinking sphere: after the step their lists need more than the storage for the
+    lists before it (half as many again), which compute_forces() has to find out."""
+    n, g = 2000, np.random.default_rng(81)
+    d = g.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1)[:, None]
+    pos, rad = (0.35 * d).astype(np.float32), np.full(n, 0.002, np.float32)
+    quiet = dict(gravity=[0.0, 0.0, 0.0], van_der_waals_strength=0.0, viscosity=0.0, damping=1.0)
+    sim = fd.FoamSimulator(pos, rad, physics=_phys(fd, **quiet))
+    sim.set_state(velocity=(-0.1 * d).astype(np.float32))
+    sim.step(1.0, 1)  # to a radius of 0.25; lists reach 0.012 + 2.5 steps of travel
+    b = sim.bubbles()
+    reach = np.array([(np.linalg.norm(p[:, None] - p[None], axis=2) < 0.262).sum() for p in (pos, b["position"])])
+    assert reach[1] > 1.6 * reach[0]
+    sim.set_physics(van_der_waals_strength=1.0)  # (a pull to see: bubbles of 2 mm are in contact here and there)
+    idx = np.arange(0, n, 7)
+    want = orc.foam_forces_subset(sim.physics, b["position"], b["radius"], idx, velocity=b["velocity"])
+    assert np.abs(want).max() > 0
+    np.testing.assert_array_equal(sim.compute_forces()[idx], want)
+    want = sim.compute_forces()
+    sim.set_state(position=b["position"])  # a list from scratch
+    np.testing.assert_array_equal(sim.compute_forces(), want)
