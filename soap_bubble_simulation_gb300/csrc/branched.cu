@@ -112,9 +112,14 @@ __device__ __forceinline__ float exp_cw_near(float x) {
     return __int_as_float(__float_as_int(p) + ((__float_as_int(t) - 0x4b400000) << 23));
 }
 
-__device__ __forceinline__ float divide(float a, float b, float r) {  // any a
-    return fabsf(a) < kTiny ? a / b : quotient(a, b, r);
+constexpr float kHuge = 0x1p90f;  // beyond it a quotient's residual may be infinity times zero
+
+__device__ __forceinline__ float divide(float a, float b, float r) {  // any a, b of ordinary size
+    return fabsf(a) < kTiny || !(fabsf(a) < kHuge) ? a / b : quotient(a, b, r);
 }
+
+// Whether quotient() may form numerators of at least `least` over b (a length, so none is larger).
+__device__ __forceinline__ bool ordinary(float least, float b) { return least >= kTiny && b >= kTiny && b < kHuge; }
 
 __device__ __forceinline__ float fract(float x) { return x - floorf(x); }
 
@@ -258,7 +263,7 @@ __global__ void __launch_bounds__(128) trace_kernel(const TraceArgs a) {
         const float qz = s.ez + s.t1z * posx + s.t2z * posy;
         const float ql = sqrtf(qx * qx + qy * qy + qz * qz);
         float nx, ny, nz;
-        if (fminf(fminf(fabsf(qx), fabsf(qy)), fabsf(qz)) < kTiny) {
+        if (!ordinary(fminf(fminf(fabsf(qx), fabsf(qy)), fabsf(qz)), ql)) {
             nx = qx / ql;
             ny = qy / ql;
             nz = qz / ql;
@@ -335,7 +340,7 @@ __global__ void __launch_bounds__(128) trace_kernel(const TraceArgs a) {
         vy = vy + ty * p.bend_strength * dt;
         const float vm = sqrtf(vx * vx + vy * vy);
         if (vm > 0.001f) {
-            if (fminf(fabsf(vx), fabsf(vy)) < kTiny) {
+            if (!ordinary(fminf(fabsf(vx), fabsf(vy)), vm)) {
                 vx = vx / vm;
                 vy = vy / vm;
             } else {

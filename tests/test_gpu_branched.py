@@ -78,3 +78,23 @@ def test_every_number_of_lanes_per_ray_matches_oracle(sbs, orc, br, rays):
     got = br.branched_flow_step(p, th, sc, tex0, fade=False)
     assert np.array_equal(got, orc.branched_flow(p, th, sc, tex0, False))
     assert got.sum() > 0
+
+
+@pytest.mark.parametrize("kw,scale", [({"bend_strength": 1e17}, 2e4), ({"bend_strength": 1e24}, 2e4),
+                                      ({"bend_strength": -1e33, "particle_weight": 0.5}, 2e4),
+                                      ({"spread_angle": 1e16}, 2e4), ({"spread_angle": 1e23}, 2e4),
+                                      ({}, 1e43), ({"step_size": 1e30}, 2e4)])
+@pytest.mark.parametrize("rays", [2000, 30000])
+def test_values_whose_squares_overflow_match_oracle(sbs, orc, br, kw, scale, rays):
+    """Velocities and positions on both sides of where a length's square is infinite: the division by
+    an infinite length gives zero, and the ray goes on."""
+    p = br.BranchedFlowParams.default()
+    p.num_rays, p.patch_enabled, p.ray_steps = rays, 0, 40
+    for k, v in kw.items():
+        setattr(p, k, v)
+    with np.errstate(over="ignore"):
+        th = field(scale=scale)
+    sc = br.generate_scatterers(p, time=1.5)
+    tex0 = np.zeros((p.tex_height, p.tex_width), np.uint32)
+    got = br.branched_flow_step(p, th, sc, tex0, fade=False)
+    assert np.array_equal(got, orc.branched_flow(p, th, sc, tex0, False))
