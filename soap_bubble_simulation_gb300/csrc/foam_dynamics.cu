@@ -1387,7 +1387,6 @@ int sbs_foam_sim_destroy(sbs_foam_sim *s) {
     cudaFree(s->split);
     cudaFree(s->perm);
     cudaFree(s->inv);
-    cudaFree(s->inv);
     cudaFree(s->mhist);
     cudaFree(s->mstart);
     cudaFree(s->gcap);

@@ -325,16 +325,3 @@ def test_forces_where_the_list_outgrows_its_storage(fd, orc):
     want = sim.compute_forces()
     sim.set_state(position=b["position"])  # a list from scratch
     np.testing.assert_array_equal(sim.compute_forces(), want)
-
-
-def test_simulators_give_their_memory_back(fd):
-    import torch
-
-    pos, rad = fd.fcc_foam(1 << 20, seed=1)
-
-    def make():
-        for _ in range(4):
-            fd.FoamSimulator(pos, rad).close()
-        return torch.cuda.mem_get_info()[0]
-
-    assert make() - make() < 8 << 20  # an index per bubble that stays behind is 16 MB
