@@ -66,8 +66,8 @@ const char *sbs_version(void);
 int sbs_device_count(int *out);
 
 /* Bounded device-side waits (no reference counterpart). Every wait inside this
- * library's kernels - the foam batch's grid barrier, the pole-ring barrier of the
- * blocked DrainageSimulator step, the mbarrier waits of the tensor-core spectral
+ * library's kernels - the foam batch's grid barrier, the pole-ring exchange of the
+ * blocked DrainageSimulator step, the resident route's row exchange, the mbarrier waits of the tensor-core spectral
  * contraction and of the fused surrogate kernel - gives up
  * after `cycles` SM clock cycles (default 2e9, about one second): the kernel
  * records the timeout, finishes its outstanding tensor-core work, frees its
@@ -82,8 +82,9 @@ int sbs_wait_limit(uint64_t *out);
  * SBS_STALL_TENSOR_COMMITS: the tensor-core kernels issue neither their MMAs
  * nor the commits that signal them, so nothing asynchronous is in flight when
  * the waits expire. SBS_STALL_GRID_BARRIER: the foam kernel's grid barrier and
- * the pole-ring barrier of the blocked DrainageSimulator step expect one arrival
- * more than there are blocks. 0 (the default) turns both off.
+ * the pole-ring exchange of the blocked DrainageSimulator step expect one arrival
+ * more than there are blocks, the resident route's row exchange a step that is
+ * never published. 0 (the default) turns both off.
  * Process-wide; meant for tests, which set a short wait limit first. */
 #define SBS_STALL_TENSOR_COMMITS 1
 #define SBS_STALL_GRID_BARRIER 2
@@ -261,22 +262,43 @@ int sbs_gpu_drainage_set_bubble_radius(sbs_drainage *h, float radius);
 int sbs_gpu_drainage_set_marangoni_enabled(sbs_drainage *h, int enabled);
 int sbs_gpu_drainage_set_marangoni_params(sbs_drainage *h, float gamma_air, float gamma_reduction,
                                           float surfactant_diffusion, float marangoni_coeff);
-/* Steps advanced per kernel launch (no reference counterpart). 2..4 use the
- * temporally blocked kernel (one read and one write of the fields per K steps;
- * choosing K needs a grid_width that is a multiple of 4), 0 or 1 launch one step
- * at a time. The results are bit-identical either way. Default 4; other widths
- * (at least 8) are blocked by default too, which time_blocking reports as 1. */
+/* How a handle's steps are launched (no reference counterpart). The fields are
+ * bit-identical on every route.
+ *  SBS_ROUTE_SINGLE    one step per launch.
+ *  SBS_ROUTE_BLOCKED   K = 2..4 steps per launch, one read and one write of the
+ *                      fields for K steps; see set_time_blocking below.
+ *  SBS_ROUTE_RESIDENT  up to 256 steps per launch, the fields held in the SMs'
+ *                      shared memory. For grids that fit there: rows of at most
+ *                      2048 columns, DrainageSimulator at most 5 rows per block.
+ *  SBS_ROUTE_AUTO      what a new handle has: resident where the grid fits,
+ *                      else blocked with the default K where it can be, else
+ *                      single steps.
+ * set_route refuses a route that the grid does not allow (SBS_E_INVALID, the
+ * route stays). BLOCKED keeps a K chosen before. route reports the route in use
+ * (never AUTO). */
+#define SBS_ROUTE_SINGLE 0
+#define SBS_ROUTE_BLOCKED 1
+#define SBS_ROUTE_RESIDENT 2
+#define SBS_ROUTE_AUTO 3
+int sbs_drainage_set_route(sbs_drainage *h, int route);
+int sbs_drainage_route(const sbs_drainage *h, int *out);
+/* Steps per blocked launch (no reference counterpart). Setting 2..4 chooses the
+ * blocked route with that K (the grid_width has to be a multiple of 4), 0 or 1
+ * the single-step route; either turns the resident route off until set_route
+ * brings it back. time_blocking reports the blocked route's K, also while the
+ * resident route is in use. Default 4; other widths (at least 8) are blocked by
+ * default too, which time_blocking reports as 1. */
 int sbs_gpu_drainage_set_time_blocking(sbs_drainage *h, int steps_per_launch);
 int sbs_gpu_drainage_time_blocking(const sbs_drainage *h, int *out);
 /* The same for a handle of either semantics (no reference counterpart). For the
  * DrainageSimulator semantics 2..4 steps per launch advance the stencil, the
  * pole-ring means and the marginal-regeneration fronts K steps at a time (row
- * strips of blocks spanning the ring, all resident at once; the two polar
- * strips meet at a bounded barrier per ring mean, see sbs_set_wait_limit); it
- * needs at least 2 (K + 1) theta rows, and choosing K an even resolution. Results
- * are bit-identical to single steps. Default where supported: 3 for the
- * compensated f32x2 storage, 4 for plain f32 (WGSL semantics: 4); odd resolutions
- * are blocked by default too, which time_blocking() reports as 1. */
+ * strips of blocks spanning the ring, all resident at once; the blocks of the
+ * two polar strips wait for each other's part of every ring mean, see
+ * sbs_set_wait_limit); it needs at least 2 (K + 1) theta rows, and choosing K an
+ * even resolution. Default where supported: 3 for the compensated f32x2 storage,
+ * 4 for plain f32 (WGSL semantics: 4); odd resolutions are blocked by default
+ * too, which time_blocking() reports as 1. */
 int sbs_drainage_set_time_blocking(sbs_drainage *h, int steps_per_launch);
 int sbs_drainage_time_blocking(const sbs_drainage *h, int *out);
 

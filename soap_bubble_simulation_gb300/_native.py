@@ -40,6 +40,7 @@ NN_ACT_HSWISH = 1
 NN_STEPS = 64
 STALL_TENSOR_COMMITS = 1
 STALL_GRID_BARRIER = 2
+ROUTES = ("single", "blocked", "resident", "auto")  # SBS_ROUTE_*
 
 _ERR_NAMES = {
     SBS_E_INVALID: "SBS_E_INVALID",
@@ -172,6 +173,8 @@ SIGNATURES: dict[str, list] = {
     "sbs_set_stall_injection": [_I],
     "sbs_drainage_set_time_blocking": [_P, _I],
     "sbs_drainage_time_blocking": [_P, _IP],
+    "sbs_drainage_set_route": [_P, _I],
+    "sbs_drainage_route": [_P, _IP],
     "sbs_gpu_drainage_set_enabled": [_P, _I],
     "sbs_gpu_drainage_set_time_scale": [_P, _F],
     "sbs_gpu_drainage_set_steps_per_frame": [_P, _U32],

@@ -217,6 +217,22 @@ int refresh(sbs_drainage *h, Consts *k) {
 
 Consts &consts_of(sbs_drainage *h) { return h->k; }
 
+// The steps per blocked launch that a new handle has, where its grid can be blocked.
+void default_blocking(sbs_drainage *h) {
+    h->wtb_k = h->cpu_k = 0;
+    if (h->sem == SBS_WGSL_SEMANTICS) {
+        if (!wtb_supported(h->nt, h->np)) return;
+        h->wtb_k = 4;
+        h->wgeom = wtb_geometry(h->nt, h->np, h->wtb_k);
+        return;
+    }
+    // steps per launch measured fastest at 2048 x 4096: 3 for the compensated storage (19.7 us
+    // per step; K = 2 20.2, K = 4 spills), 4 for plain f32 (10.7 us)
+    const int k = h->x2 ? 3 : 4;
+    h->cgeom = wtbc_geometry(h->nt, h->np, k, h->x2);
+    if (h->cgeom.nby > 0) h->cpu_k = k;
+}
+
 int allocate(sbs_drainage *h) {
     const size_t bytes = h->pitch * (size_t)h->nt * sizeof(float);
     SBS_CUDA_TRY(cudaGetDevice(&h->device));
@@ -234,18 +250,8 @@ int allocate(sbs_drainage *h) {
         }
     }
     h->geom = step_geometry(h->nt, h->np, h->sem, h->x2);
-    if (h->sem == SBS_WGSL_SEMANTICS && wtb_supported(h->nt, h->np)) {
-        h->wtb_k = 4;
-        h->wgeom = wtb_geometry(h->nt, h->np, h->wtb_k);
-        h->cau_geom = wtb_geometry(h->nt, h->np, kWtbCausticK);
-    }
-    if (h->sem == SBS_CPU_SEMANTICS) {
-        // steps per launch measured fastest at 2048 x 4096: 3 for the compensated storage (19.7 us
-        // per step; K = 2 20.2, K = 4 spills), 4 for plain f32 (10.7 us)
-        const int k = h->x2 ? 3 : 4;
-        h->cgeom = wtbc_geometry(h->nt, h->np, k, h->x2);
-        if (h->cgeom.nby > 0) h->cpu_k = k;
-    }
+    default_blocking(h);
+    if (h->wtb_k > 1) h->cau_geom = wtb_geometry(h->nt, h->np, kWtbCausticK);
     h->rgeom = resident_geometry(h->nt, h->np, h->sem, h->x2);
     h->resident = h->rgeom.nby > 0;
     // one volume partial per block of whichever step kernel runs the check
@@ -1306,6 +1312,32 @@ int sbs_drainage_time_blocking(const sbs_drainage *h, int *out) {
     SBS_CHECK_ARG(out != nullptr, "out is null");
     if (h->sem == SBS_WGSL_SEMANTICS) return sbs_gpu_drainage_time_blocking(h, out);
     *out = blocking_selectable(h) && h->cpu_k > 1 ? h->cpu_k : 1;
+    return SBS_OK;
+}
+
+int sbs_drainage_set_route(sbs_drainage *h, int route) {
+    clear_error();
+    CHECK_HANDLE(h);
+    SBS_CHECK_ARG(route >= SBS_ROUTE_SINGLE && route <= SBS_ROUTE_AUTO, "bad route %d", route);
+    const bool fits = h->rgeom.nby > 0;
+    if (route == SBS_ROUTE_RESIDENT && !fits)
+        return set_error(SBS_E_INVALID, "a grid of %d x %d does not fit the chip", h->nt, h->np);
+    SBS_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    if (route == SBS_ROUTE_SINGLE)
+        h->wtb_k = h->cpu_k = 0;
+    else if (route != SBS_ROUTE_BLOCKED || (h->wtb_k < 2 && h->cpu_k < 2))
+        default_blocking(h);
+    if (route == SBS_ROUTE_BLOCKED && h->wtb_k < 2 && h->cpu_k < 2)
+        return set_error(SBS_E_INVALID, "a grid of %d x %d is too small for blocked steps", h->nt, h->np);
+    destroy_graphs(h);
+    h->resident = fits && (route == SBS_ROUTE_RESIDENT || route == SBS_ROUTE_AUTO);
+    return SBS_OK;
+}
+
+int sbs_drainage_route(const sbs_drainage *h, int *out) {
+    CHECK_HANDLE(h);
+    SBS_CHECK_ARG(out != nullptr, "out is null");
+    *out = h->resident ? SBS_ROUTE_RESIDENT : h->wtb_k > 1 || h->cpu_k > 1 ? SBS_ROUTE_BLOCKED : SBS_ROUTE_SINGLE;
     return SBS_OK;
 }
 

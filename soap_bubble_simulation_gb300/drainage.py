@@ -205,6 +205,21 @@ class _Handle:
         N.call("sbs_drainage_run_checked", self.handle, float(dt), int(n), int(check_every), N.dptr(vols))
         return vols[:k]
 
+    @property
+    def route(self) -> str:
+        """How steps are launched: "single", "blocked" (2 to 4 steps per launch) or "resident" (up to 256
+        steps per launch, for grids that fit the chip). Setting "auto" gives what a new simulator has. The
+        results are the same bits on every route."""
+        out = C.c_int()
+        N.call("sbs_drainage_route", self.handle, C.byref(out))
+        return N.ROUTES[out.value]
+
+    @route.setter
+    def route(self, v: str) -> None:
+        if v not in N.ROUTES:
+            raise ValueError(f"route must be one of {N.ROUTES}")
+        N.call("sbs_drainage_set_route", self.handle, N.ROUTES.index(v))
+
     def stream(self) -> int:
         out = C.c_void_p()
         N.call("sbs_drainage_stream", self.handle, C.byref(out))

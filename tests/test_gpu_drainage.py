@@ -655,3 +655,55 @@ def test_resident_cpu_chunks_match_single_steps(sbs, precision, res):
     np.testing.assert_array_equal(out[0][0], out[1][0])
     np.testing.assert_allclose(out[0][1], out[1][1], rtol=1e-12)
     assert out[0][2] == out[1][2] >= 1
+
+
+@pytest.mark.parametrize("semantics,nt,np_,routes", [
+    ("wgsl", 64, 128, ("resident", "blocked", "single")), ("wgsl", 33, 131, ("resident", "blocked", "single")),
+    ("wgsl", 3, 7, ("resident", "single")), ("wgsl", 40, 2052, ("blocked", "single")),
+    ("wgsl", 40, 2051, ("blocked", "single")), ("cpu", 64, 128, ("resident", "blocked", "single")),
+    ("cpu", 61, 122, ("resident", "blocked", "single")), ("cpu", 4, 8, ("resident", "single")),
+    ("cpu", 1026, 2052, ("blocked", "single"))])
+def test_routes_are_chosen_and_reported(sbs, semantics, nt, np_, routes):
+    """Every route that a grid allows, from any other, in the middle of a run: the same bits; a route that
+    it does not allow is refused and leaves the one in use."""
+    from soap_bubble_simulation_gb300 import synthetic
+
+    def make():
+        if semantics == "cpu":
+            return make_sim(sbs, nt)
+        sim = sbs.GPUDrainageSimulator(None, 500e-9, np_, nt)
+        sim.set_thickness_array(synthetic.smooth_modes(nt, np_, seed=nt).astype(np.float32))
+        return sim
+
+    def run(sim, n):
+        sim.step_n(1e-4, n) if semantics == "cpu" else sim.run(n)
+
+    sim, ref = make(), make()
+    ref.route = "single"
+    assert sim.route == routes[0] and ref.route == "single"
+    for route in ("blocked", "auto", "single", "resident", "blocked", "single", "auto"):
+        before = sim.route
+        if route == "auto" or route in routes:
+            sim.route = route
+            assert sim.route == (routes[0] if route == "auto" else route)
+        else:
+            with pytest.raises(sbs.SbsError, match="fit|small"):
+                sim.route = route
+            assert sim.route == before
+        run(sim, 13)
+        run(ref, 13)
+        np.testing.assert_array_equal(sim.thickness_array(), ref.thickness_array())
+    with pytest.raises(ValueError):
+        sim.route = "fast"
+    out = ctypes.c_int()
+    sbs._native.call("sbs_drainage_time_blocking", sim.handle, ctypes.byref(out))
+    if np_ % 4 == 0 and "blocked" in routes:  # a chosen K leaves the resident route, and stays until "auto"
+        set_cpu_blocking(sbs, sim, 2)
+        assert sim.route == "blocked"
+        sim.route = "blocked"
+        assert cpu_blocking(sbs, sim) == 2
+        sim.route = "auto"
+        assert sim.route == routes[0] and cpu_blocking(sbs, sim) == out.value
+    run(sim, 13)
+    run(ref, 13)
+    np.testing.assert_array_equal(sim.thickness_array(), ref.thickness_array())
