@@ -217,13 +217,17 @@ int refresh(sbs_drainage *h, Consts *k) {
 
 Consts &consts_of(sbs_drainage *h) { return h->k; }
 
+void block_wgsl(sbs_drainage *h, int K) {
+    h->wtb_k = K;
+    for (int mar = 0; mar < 2; ++mar) h->wgeom[mar] = wtb_geometry(h->nt, h->np, K, mar != 0);
+}
+
 // The steps per blocked launch that a new handle has, where its grid can be blocked.
 void default_blocking(sbs_drainage *h) {
     h->wtb_k = h->cpu_k = 0;
     if (h->sem == SBS_WGSL_SEMANTICS) {
         if (!wtb_supported(h->nt, h->np)) return;
-        h->wtb_k = 4;
-        h->wgeom = wtb_geometry(h->nt, h->np, h->wtb_k);
+        block_wgsl(h, 4);
         return;
     }
     // steps per launch measured fastest at 2048 x 4096: 3 for the compensated storage (19.7 us
@@ -251,16 +255,14 @@ int allocate(sbs_drainage *h) {
     }
     h->geom = step_geometry(h->nt, h->np, h->sem, h->x2);
     default_blocking(h);
-    if (h->wtb_k > 1) h->cau_geom = wtb_geometry(h->nt, h->np, kWtbCausticK);
+    if (h->wtb_k > 1)
+        for (int mar = 0; mar < 2; ++mar) h->cau_geom[mar] = wtb_geometry(h->nt, h->np, kWtbCausticK, mar != 0);
     h->rgeom = resident_geometry(h->nt, h->np, h->sem, h->x2);
     h->resident = h->rgeom.nby > 0;
     // one volume partial per block of whichever step kernel runs the check
     size_t vol_blocks = (size_t)h->geom.nbx * h->geom.nby;
     if (h->sem == SBS_WGSL_SEMANTICS && wtb_supported(h->nt, h->np))
-        for (int k = 2; k <= 4; ++k) {
-            const StepGeom g = wtb_geometry(h->nt, h->np, k);
-            vol_blocks = std::max(vol_blocks, (size_t)g.nbx * g.nby);
-        }
+        vol_blocks = std::max(vol_blocks, (size_t)h->wgeom[0].nbx * h->nt);  // whatever K and Marangoni make of it
     vol_blocks = std::max(vol_blocks, (size_t)h->rgeom.nby);
     size_t slots = 0;
     if (h->sem == SBS_CPU_SEMANTICS)
@@ -348,7 +350,7 @@ bool blocking_selectable(const sbs_drainage *h) { return h->np % 4 == 0; }
 // single pass (the map is of the field one pass behind the newest, the buffer the renderer binds).
 bool cau_plan(const sbs_drainage *h, int count, bool last_single) {
     return h->cau_on && h->sem == SBS_WGSL_SEMANTICS && !h->resident && h->wtb_k > 1 && last_single &&
-           h->cau_geom.nby > 0 && count - 1 >= kWtbCausticK;
+           h->cau_geom[0].nby > 0 && count - 1 >= kWtbCausticK;
 }
 
 // The bounded waits' limit and status words, the test switch that makes them run out, and the ring's
@@ -509,7 +511,9 @@ int enqueue_steps(sbs_drainage *h, int start, int count, float dt, bool vol_last
         a.pitch = (int)h->pitch;
         const bool cau_launch = plan[i] < 0;
         const int steps = cau_launch ? -plan[i] : plan[i];
-        a.rb = cau_launch ? h->cau_geom.rb : steps > 1 ? h->wgeom.rb : h->geom.rb;
+        const int mar = h->params.marangoni_enabled ? 1 : 0;
+        const StepGeom &wg = cau_launch ? h->cau_geom[mar] : h->wgeom[mar];
+        a.rb = steps > 1 ? wg.rb : h->geom.rb;
         if (cau_launch) {
             a.cau_out = h->cau_out;
             a.cau_focal = h->cau_p[0];
@@ -518,7 +522,7 @@ int enqueue_steps(sbs_drainage *h, int start, int count, float dt, bool vol_last
             a.cau_branch = h->cau_p[3];
         }
         a.poles_virtual = i > 0 ? 1 : 0;
-        a.marangoni = h->params.marangoni_enabled ? 1 : 0;
+        a.marangoni = mar;
         a.crit = k.crit;
         a.b = k.b;
         a.DR2 = k.DR2;
@@ -527,7 +531,7 @@ int enqueue_steps(sbs_drainage *h, int start, int count, float dt, bool vol_last
         a.M = k.M;
         a.dt = dt;
         if (steps > 1)
-            SBS_CUDA_TRY(launch_wtb(steps, a, cau_launch ? h->cau_geom : h->wgeom, h->stream));
+            SBS_CUDA_TRY(launch_wtb(steps, a, wg, h->stream));
         else
             SBS_CUDA_TRY(launch_step(h->sem, h->x2, a, h->geom, h->stream));
         cur ^= 1;
@@ -1274,8 +1278,8 @@ int sbs_gpu_drainage_set_time_blocking(sbs_drainage *h, int steps_per_launch) {
         return set_error(SBS_E_INVALID, "time blocking needs grid_width a multiple of 4 (got %d)", h->np);
     destroy_graphs(h);
     h->resident = false;
-    h->wtb_k = steps_per_launch > 1 ? steps_per_launch : 0;
-    if (h->wtb_k) h->wgeom = wtb_geometry(h->nt, h->np, h->wtb_k);
+    h->wtb_k = 0;
+    if (steps_per_launch > 1) block_wgsl(h, steps_per_launch);
     return SBS_OK;
 }
 

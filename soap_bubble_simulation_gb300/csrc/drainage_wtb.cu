@@ -18,6 +18,8 @@
 // launches of one and one launch of this give bit-identical fields.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "cell.cuh"
 #include "sbs_internal.h"
 #include "wtb.cuh"
@@ -173,7 +175,10 @@ bool wtb_supported(int nt, int np) { return np >= 8 && nt >= 3; }
 // K levels are a chain) and 0.3 us more for every further one (issue). Measured per pass at
 // K = 4, against strips of at least 16 rows that fill three blocks per SM: 64 x 128 3.1 -> 1.5 us (one row),
 // 256 x 512 3.3 -> 2.0, 512 x 1024 3.5 -> 2.8, 1024 x 2048 5.8 -> 5.2; 2048 x 4096 keeps its 41 rows.
-StepGeom wtb_geometry(int nt, int np, int K) {
+// Marangoni's chain is longer (its roots): an iteration takes 1.1 us with one warp and with two, 1.45 with
+// three. Weighed with the plain times, 500 x 2501 took 8.9 us a pass and 1025 x 2051 13.9 (single steps
+// 7.0 and 12.6); with these 5.9 and 8.7 (500 x 2500: 8.2, 5.5).
+StepGeom wtb_geometry(int nt, int np, int K, bool mar) {
     StepGeom g{};
     const int segs = (np + kSegStride - 1) / kSegStride;
     g.nbx = (segs + kWarpsPerBlock - 1) / kWarpsPerBlock;
@@ -181,7 +186,7 @@ StepGeom wtb_geometry(int nt, int np, int K) {
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wtb_kernel(K, np % 4 != 0, false, false), g.wx * 32,
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wtb_kernel(K, np % 4 != 0, false, mar), g.wx * 32,
                                                   wtb_smem(g.wx, 64, K, false));
     if (per_sm < 1) per_sm = 1;
     double best = 0.0;
@@ -189,7 +194,7 @@ StepGeom wtb_geometry(int nt, int np, int K) {
         const long long blocks = (long long)g.nbx * ((nt - 2 + rb - 1) / rb);
         const long long each = (blocks + sms - 1) / sms, waves = (each + per_sm - 1) / per_sm;  // per SM
         const double warps = (double)(waves > 1 ? per_sm : each) * g.wx / 4.0;                  // per scheduler
-        const double iteration = warps > 0.9 ? 0.14 + 0.3 * warps : 0.41;
+        const double iteration = mar ? std::max(1.1, 0.48 * warps) : warps > 0.9 ? 0.14 + 0.3 * warps : 0.41;
         const double cost = waves * (2.5 + (rb + 2 * K) * iteration);
         if (rb == 1 || cost < best) {
             best = cost;

@@ -126,7 +126,7 @@ struct StepGeom {
 StepGeom step_geometry(int nt, int np, int semantics, int x2);
 // Temporally blocked WGSL step (K = 2..4 steps per launch), drainage_wtb.cu.
 bool wtb_supported(int nt, int np);
-StepGeom wtb_geometry(int nt, int np, int K);
+StepGeom wtb_geometry(int nt, int np, int K, bool mar);
 cudaError_t launch_wtb(int K, const StepArgs &a, const StepGeom &g, cudaStream_t s);
 // K for a launch that also writes the caustic map of its result (a.cau_out): its final level must
 // leave one valid column beyond the kept 120 on each side of a warp's window.
@@ -258,7 +258,7 @@ struct sbs_drainage {
     size_t qcap = 0;
     sbs::StepGeom geom{};
     int wtb_k = 0;  // steps per temporally blocked launch (WGSL semantics; 0 = single steps only)
-    sbs::StepGeom wgeom{};
+    sbs::StepGeom wgeom[2]{};          // without and with Marangoni
     int cpu_k = 0;  // steps per temporally blocked launch (CPU semantics; 0 = single steps only)
     sbs::StepGeom cgeom{};
     bool resident = false;                     // chunks run through the resident kernel
@@ -276,7 +276,7 @@ struct sbs_drainage {
     float *cau_out = nullptr;          // device destination of the map
     float cau_p[4] = {0.f, 0.f, 0.f, 0.f};  // focal length, intensity, sharpness, branch threshold
     float *cau_buf = nullptr;          // device map for calls with host memory
-    sbs::StepGeom cau_geom{};          // geometry of the launch that writes the map
+    sbs::StepGeom cau_geom[2]{};       // geometry of the launch that writes the map, likewise
 
     // CPU semantics parameters (from sbs_config)
     sbs_config cfg{};

@@ -707,3 +707,28 @@ def test_routes_are_chosen_and_reported(sbs, semantics, nt, np_, routes):
     run(sim, 13)
     run(ref, 13)
     np.testing.assert_array_equal(sim.thickness_array(), ref.thickness_array())
+
+
+@pytest.mark.parametrize("W,H", [(2051, 200), (2500, 121), (2501, 500), (8, 30)])
+def test_marangoni_strips_match_single_steps(sbs, W, H):
+    """Blocked steps with Marangoni, whose strips have their own height, and the plain ones of the same
+    handle: single steps' bits, volumes, the shorter launches of a remainder."""
+    from soap_bubble_simulation_gb300 import synthetic
+
+    h = synthetic.smooth_modes(H, W, seed=W + H).astype(np.float32)
+    c = synthetic.surfactant_noise(H, W, seed=H)
+    out = []
+    for route in ("blocked", "single"):
+        sim = sbs.GPUDrainageSimulator(None, 500e-9, W, H)
+        sim.route = route
+        sim.set_thickness_array(h)
+        sim.set_concentration_array(c)
+        vols = []
+        for marangoni in (1, 0, 1):
+            sim.set_marangoni_enabled(bool(marangoni))
+            vols.append(sim.run_checked(0.0, 22, 11))
+            sim.run(4)
+        out.append((sim.thickness_array(), sim.concentration_array(), np.concatenate(vols)))
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+    np.testing.assert_allclose(out[0][2], out[1][2], rtol=1e-12)
