@@ -270,9 +270,11 @@ int sbs_gpu_drainage_set_marangoni_params(sbs_drainage *h, float gamma_air, floa
  *  SBS_ROUTE_RESIDENT  up to 256 steps per launch, the fields held in the SMs'
  *                      shared memory. For grids that fit there: rows of at most
  *                      2048 columns, DrainageSimulator at most 5 rows per block.
- *  SBS_ROUTE_AUTO      what a new handle has: resident where the grid fits,
- *                      else blocked with the default K where it can be, else
- *                      single steps.
+ *  SBS_ROUTE_AUTO      what a new handle has: resident where the grid fits
+ *                      (route reports that; runs of a few passes of a large grid
+ *                      are launched as the blocked route does, where that is
+ *                      faster), else blocked with the default K where it can
+ *                      be, else single steps.
  * set_route refuses a route that the grid does not allow (SBS_E_INVALID, the
  * route stays). BLOCKED keeps a K chosen before. route reports the route in use
  * (never AUTO). */

@@ -237,6 +237,30 @@ void default_blocking(sbs_drainage *h) {
     if (h->cgeom.nby > 0) h->cpu_k = k;
 }
 
+// Whether a chunk of `count` steps runs in the resident kernel. It pays the field's way into shared
+// memory and back (and the launch of resident blocks) once a chunk, so few WGSL passes of a large grid
+// are left to the other kernels (resident_from).
+bool use_resident(const sbs_drainage *h, int count) {
+    return h->resident && count >= h->res_min[h->sem == SBS_WGSL_SEMANTICS && h->params.marangoni_enabled ? 1 : 0];
+}
+
+// The fewest steps of a chunk that the resident kernel runs by default. DrainageSimulator: any number
+// (one step of 128 x 256 16 us a call, 24 in the single-step kernel; 700 x 1400 23 and 27). WGSL, us a
+// call resident / otherwise: one pass 64 x 128 14.0 / 12.7, 1024 x 2048 20.8 / 16.8, 1500 x 1500 26.4 / 17.4;
+// more plain passes 517 x 1037 two 21.4 / 21.7; 900 x 1800 five 36.5 / 35.9, six 39.8 / 44.2; 1300 x 2000
+// twelve 80.3 / 75.9, 48 253 / 262; 2000 x 1600 48 335 / 310, 256 1659 / 1589. With Marangoni, whose single
+// steps and blocked launches are slower, 1500 x 1500 two 35.8 / 34.0, four 46.8 / 47.2, 48 299 / 419.
+void resident_from(sbs_drainage *h) {
+    h->res_min[0] = h->res_min[1] = 1;
+    if (h->sem != SBS_WGSL_SEMANTICS) return;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long long cells = (long long)h->nt * h->np / sms;  // an SM's share
+    h->res_min[0] = cells <= 8000 ? 2 : cells <= 17000 ? 6 : cells <= 19000 ? 16 : kMaxChunk + 1;
+    h->res_min[1] = cells <= 8000 ? 2 : 3;
+}
+
 int allocate(sbs_drainage *h) {
     const size_t bytes = h->pitch * (size_t)h->nt * sizeof(float);
     SBS_CUDA_TRY(cudaGetDevice(&h->device));
@@ -259,6 +283,7 @@ int allocate(sbs_drainage *h) {
         for (int mar = 0; mar < 2; ++mar) h->cau_geom[mar] = wtb_geometry(h->nt, h->np, kWtbCausticK, mar != 0);
     h->rgeom = resident_geometry(h->nt, h->np, h->sem, h->x2);
     h->resident = h->rgeom.nby > 0;
+    resident_from(h);
     // one volume partial per block of whichever step kernel runs the check
     size_t vol_blocks = (size_t)h->geom.nbx * h->geom.nby;
     if (h->sem == SBS_WGSL_SEMANTICS && wtb_supported(h->nt, h->np))
@@ -349,7 +374,7 @@ bool blocking_selectable(const sbs_drainage *h) { return h->np % 4 == 0; }
 // the final chunk of a run that asked for the map, blocked, with three passes before the final
 // single pass (the map is of the field one pass behind the newest, the buffer the renderer binds).
 bool cau_plan(const sbs_drainage *h, int count, bool last_single) {
-    return h->cau_on && h->sem == SBS_WGSL_SEMANTICS && !h->resident && h->wtb_k > 1 && last_single &&
+    return h->cau_on && h->sem == SBS_WGSL_SEMANTICS && !use_resident(h, count) && h->wtb_k > 1 && last_single &&
            h->cau_geom[0].nby > 0 && count - 1 >= kWtbCausticK;
 }
 
@@ -584,7 +609,7 @@ int run_chunk(sbs_drainage *h, int count, double dt, bool vol_last, bool last_si
         for (int i = 0; i < count; ++i) h->current_time += (double)h->params.dt;
     }
     int end = h->cur;
-    if (h->resident) {
+    if (use_resident(h, count)) {
         int rc = enqueue_resident(h, count, dtf, vol_last, use_sched);
         if (rc) return rc;
         end = h->cur ^ 1;
@@ -1335,6 +1360,8 @@ int sbs_drainage_set_route(sbs_drainage *h, int route) {
         return set_error(SBS_E_INVALID, "a grid of %d x %d is too small for blocked steps", h->nt, h->np);
     destroy_graphs(h);
     h->resident = fits && (route == SBS_ROUTE_RESIDENT || route == SBS_ROUTE_AUTO);
+    resident_from(h);
+    if (route == SBS_ROUTE_RESIDENT) h->res_min[0] = h->res_min[1] = 1;
     return SBS_OK;
 }
 

@@ -262,6 +262,7 @@ struct sbs_drainage {
     int cpu_k = 0;  // steps per temporally blocked launch (CPU semantics; 0 = single steps only)
     sbs::StepGeom cgeom{};
     bool resident = false;                     // chunks run through the resident kernel
+    int res_min[2] = {1, 1};                   // of at least so many steps, without and with Marangoni
     sbs::StepGeom rgeom{};
     unsigned long long *halo = nullptr;        // its row exchange
     unsigned halo_tag = 0;                     // the last step number used there

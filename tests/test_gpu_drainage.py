@@ -732,3 +732,35 @@ def test_marangoni_strips_match_single_steps(sbs, W, H):
     np.testing.assert_array_equal(out[0][0], out[1][0])
     np.testing.assert_array_equal(out[0][1], out[1][1])
     np.testing.assert_allclose(out[0][2], out[1][2], rtol=1e-12)
+
+
+@pytest.mark.parametrize("marangoni", [0, 1])
+@pytest.mark.parametrize("W,H", [(7, 3), (128, 64), (1037, 517), (1501, 900), (1999, 1300), (1600, 2000)])
+def test_runs_of_few_passes_match_single_steps(sbs, W, H, marangoni):
+    """Runs on both sides of the numbers of passes from which the resident kernel takes them, on grids of
+    every class of that rule: bits, the field one pass behind the newest, volumes, the caustic map."""
+    from soap_bubble_simulation_gb300 import synthetic
+
+    h = synthetic.smooth_modes(H, W, seed=W + H).astype(np.float32)
+    c = synthetic.surfactant_noise(H, W, seed=H)
+    out = []
+    for route in ("auto", "resident", "single"):
+        sim = sbs.GPUDrainageSimulator(None, 500e-9, W, H)
+        sim.route = route
+        assert sim.route == ("single" if route == "single" else "resident")
+        sim.set_thickness_array(h)
+        sim.set_concentration_array(c)
+        sim.set_marangoni_enabled(bool(marangoni))
+        behind = []
+        for k in (1, 2, 3, 5, 6, 15, 16):
+            sim.run(k)
+            stale = sim.current_buffer()
+            behind.append(sbs.film_volume_device(stale.ptr, H, W, stale.pitch, 0.025))
+        vols = sim.run_checked(0.0, 24, 6)
+        cau = sim.run_caustic_map(5)
+        out.append((sim.thickness_array(), sim.concentration_array(), cau, vols, behind))
+    for got in out[:2]:
+        for a, b in zip(got[:3], out[2][:3]):
+            np.testing.assert_array_equal(a, b)
+        np.testing.assert_allclose(got[3], out[2][3], rtol=1e-12)
+        np.testing.assert_allclose(got[4], out[2][4], rtol=1e-12)
