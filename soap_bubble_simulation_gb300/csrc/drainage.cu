@@ -265,18 +265,6 @@ int allocate(sbs_drainage *h) {
     const size_t bytes = h->pitch * (size_t)h->nt * sizeof(float);
     SBS_CUDA_TRY(cudaGetDevice(&h->device));
     SBS_CUDA_TRY(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
-    for (int i = 0; i < 2; ++i) {
-        SBS_CUDA_TRY(cudaMalloc(&h->h[i], bytes));
-        SBS_CUDA_TRY(cudaMemsetAsync(h->h[i], 0, bytes, h->stream));
-        if (h->sem == SBS_WGSL_SEMANTICS) {
-            SBS_CUDA_TRY(cudaMalloc(&h->c[i], bytes));
-            SBS_CUDA_TRY(cudaMemsetAsync(h->c[i], 0, bytes, h->stream));
-        }
-        if (h->x2) {
-            SBS_CUDA_TRY(cudaMalloc(&h->hl[i], bytes));
-            SBS_CUDA_TRY(cudaMemsetAsync(h->hl[i], 0, bytes, h->stream));
-        }
-    }
     h->geom = step_geometry(h->nt, h->np, h->sem, h->x2);
     default_blocking(h);
     if (h->wtb_k > 1)
@@ -298,15 +286,19 @@ int allocate(sbs_drainage *h) {
         }
     h->ring_bytes = slots + sizeof(unsigned long long);
     h->sched_cap = kMaxChunk;
-    // The small buffers are pieces of one device and one pinned allocation: a handle of some 64 x 128
-    // with its first fields took 1.06 ms to make with one each, about 0.8 with these.
+    // Fields and small buffers are pieces of one device and one pinned allocation: each that the driver
+    // maps for itself (2 MB and more) costs 60 us to make and give back. A handle of 512 x 1024 took 876 us
+    // to make and destroy with its fields apart, 628 with this; 1024 x 2048 936, 680; 64 x 128 524, 500.
     size_t dev_bytes = 0, host_bytes = 0;
     const auto piece = [](size_t &at, size_t n) {
         const size_t o = at;
         at += (n + 255) / 256 * 256;
         return o;
     };
-    const size_t o_halo = piece(dev_bytes, h->resident ? resident_halo_bytes(h->rgeom) : 0);
+    const bool second = h->sem == SBS_WGSL_SEMANTICS || h->x2;  // the surfactant, or the low words
+    const size_t o_h[2] = {piece(dev_bytes, bytes), piece(dev_bytes, bytes)};
+    const size_t o_s[2] = {piece(dev_bytes, second ? bytes : 0), piece(dev_bytes, second ? bytes : 0)};
+    const size_t o_halo = piece(dev_bytes, h->resident ? resident_halo_bytes(h->rgeom, second) : 0);
     const size_t o_part[2] = {piece(dev_bytes, sizeof(FixSum) * 2 * h->geom.nbx),
                               piece(dev_bytes, sizeof(FixSum) * 2 * h->geom.nbx)};
     const size_t o_rows = piece(dev_bytes, sizeof(float4) * h->nt), o_vol_w = piece(dev_bytes, sizeof(double) * h->nt);
@@ -315,9 +307,13 @@ int allocate(sbs_drainage *h) {
     const size_t o_red = piece(dev_bytes, sizeof(double) * 3 * reduce_partials_count(h->nt, h->np));
     const size_t o_red_count = piece(dev_bytes, sizeof(unsigned)), o_red_out = piece(dev_bytes, sizeof(ReduceOut));
     const size_t o_sched = piece(dev_bytes, sizeof(TfeStep) * h->sched_cap);
-    SBS_CUDA_TRY(cudaMalloc(&h->small, dev_bytes));
-    SBS_CUDA_TRY(cudaMemsetAsync(h->small, 0, dev_bytes, h->stream));
-    char *d = static_cast<char *>(h->small);
+    SBS_CUDA_TRY(cudaMalloc(&h->arena, dev_bytes));
+    SBS_CUDA_TRY(cudaMemsetAsync(h->arena, 0, dev_bytes, h->stream));
+    char *d = static_cast<char *>(h->arena);
+    for (int i = 0; i < 2; ++i) {
+        h->h[i] = reinterpret_cast<float *>(d + o_h[i]);
+        if (second) (h->x2 ? h->hl : h->c)[i] = reinterpret_cast<float *>(d + o_s[i]);
+    }
     if (h->resident) h->halo = reinterpret_cast<unsigned long long *>(d + o_halo);
     for (int i = 0; i < 2; ++i) h->part[i] = reinterpret_cast<FixSum *>(d + o_part[i]);
     h->rows = reinterpret_cast<float4 *>(d + o_rows);
@@ -351,15 +347,11 @@ int allocate(sbs_drainage *h) {
 void release(sbs_drainage *h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     destroy_graphs(h);
-    for (int i = 0; i < 2; ++i) {
-        cudaFree(h->h[i]);
-        cudaFree(h->c[i]);
-        cudaFree(h->hl[i]);
+    for (int i = 0; i < 2; ++i)
         if (h->sched_ev[i]) cudaEventDestroy(h->sched_ev[i]);
-    }
     cudaFree(h->vol_out);
     cudaFree(h->qbuf);
-    cudaFree(h->small);
+    cudaFree(h->arena);
     cudaFree(h->cau_buf);
     if (h->pinned) cudaFreeHost(h->pinned);
     if (h->stream) cudaStreamDestroy(h->stream);
