@@ -98,3 +98,20 @@ def test_values_whose_squares_overflow_match_oracle(sbs, orc, br, kw, scale, ray
     tex0 = np.zeros((p.tex_height, p.tex_width), np.uint32)
     got = br.branched_flow_step(p, th, sc, tex0, fade=False)
     assert np.array_equal(got, orc.branched_flow(p, th, sc, tex0, False))
+
+
+@pytest.mark.parametrize("scatterers,clustered", [(0, 0), (1, 0), (12, 0), (40, 8), (40, 9), (60, 33)])
+@pytest.mark.parametrize("rays", [500, 25000])
+def test_short_lists_match_oracle(sbs, orc, br, rays, scatterers, clustered):
+    """Lists of no scatterers up to both sides of the length that is walked without masks."""
+    p = br.BranchedFlowParams.default()
+    p.num_rays, p.patch_enabled, p.ray_steps, p.num_scatterers = rays, 0, 60, scatterers
+    sc = br.generate_scatterers(p, time=0.5)
+    if clustered:  # `clustered` of them share a cell, the others one far away
+        g = np.random.default_rng(clustered)
+        sc[:clustered, :2] = 0.72 + 0.06 * g.random((clustered, 2))
+        sc[clustered:, :2] = 0.03 + 0.005 * np.arange(scatterers - clustered)[:, None] * np.array([[0.0, 1.0]])
+    th = field(scale=2e4)
+    tex0 = np.zeros((p.tex_height, p.tex_width), np.uint32)
+    got = br.branched_flow_step(p, th, sc, tex0, fade=False)
+    assert np.array_equal(got, orc.branched_flow(p, th, sc, tex0, False))
