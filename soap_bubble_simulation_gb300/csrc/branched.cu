@@ -614,7 +614,12 @@ int sbs_branched_flow(const sbs_branched_params *p, const float *thickness, uint
         const int lanes = lanes_per_ray(p->num_rays);
         const void *fn = lanes == 1 ? (const void *)trace_kernel<1>
                          : lanes == 2 ? (const void *)trace_kernel<2> : (const void *)trace_kernel<4>;
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // always the device's limit: the attribute is the process's, and a call with fewer scatterers on
+        // another thread must not lower it between here and the launch
+        int dev = 0, most = 0;
+        e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         if (e == cudaSuccess) {
             void *args[] = {(void *)&a};
             const unsigned per_block = 128u / (unsigned)lanes;

@@ -115,3 +115,24 @@ def test_short_lists_match_oracle(sbs, orc, br, rays, scatterers, clustered):
     tex0 = np.zeros((p.tex_height, p.tex_width), np.uint32)
     got = br.branched_flow_step(p, th, sc, tex0, fade=False)
     assert np.array_equal(got, orc.branched_flow(p, th, sc, tex0, False))
+
+
+def test_threads_with_different_numbers_of_scatterers(sbs, br):
+    """Calls of several threads whose blocks want different amounts of shared memory."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    th = field(scale=2e4)
+
+    def run(n, times=1):
+        p = br.BranchedFlowParams.default()
+        p.num_rays, p.patch_enabled, p.ray_steps, p.num_scatterers = 300, 0, 5, n
+        sc = br.generate_scatterers(p, time=0.5)
+        return [br.branched_flow_step(p, th, sc, np.zeros((p.tex_height, p.tex_width), np.uint32), fade=False)
+                for _ in range(times)]
+
+    sizes = (0, 400, 1200, 2000)
+    want = [run(n)[0] for n in sizes]
+    with ThreadPoolExecutor(4) as pool:
+        for got, w in zip(pool.map(lambda n: run(n, 40), sizes), want):
+            for t in got:
+                np.testing.assert_array_equal(t, w)
