@@ -148,3 +148,57 @@ def test_step_caustic_map_fused_equals_separate_pass(sbs, cp):
     b.enabled = False
     np.testing.assert_array_equal(a.step_caustic_map(1.0 / 60.0, p), b.caustic_map(p, which=1))
     assert a.current_time() == b.current_time()
+
+
+@pytest.mark.parametrize("nt,np_,marangoni", [(10, 40, False), (37, 132, True), (33, 131, True), (130, 600, False),
+                                              (256, 512, True), (40, 2052, True), (40, 2051, False)])
+def test_fused_caustic_map_on_the_blocked_route(sbs, orc, cp, nt, np_, marangoni):
+    """The final blocked launch writes the map (rows of more than 2048 columns do so by default): the map
+    and the fields of run() and the separate pass, and of single steps, bit for bit, for every remainder
+    before that launch and over several chunks."""
+    from soap_bubble_simulation_gb300 import synthetic as S
+
+    h0 = S.smooth_modes(nt, np_, seed=nt).astype(np.float32)
+    c0 = S.surfactant_noise(nt, np_, seed=nt + 1)
+    p = _vivid(cp, np_, nt)
+    sims = []
+    for route in ("blocked", "blocked", "single"):
+        sim = sbs.GPUDrainageSimulator(None, 500e-9, np_, nt)
+        params = sbs.field_params(nt, np_, bubble_radius=0.02)
+        params.marangoni_enabled = 1 if marangoni else 0
+        sim.update_params(params)
+        sim.route = route
+        sim.set_thickness_array(h0)
+        sim.set_concentration_array(c0)
+        sims.append(sim)
+    fused, sep, single = sims
+    for passes in (3, 4, 5, 6, 7, 8, 9, 12, 300, 259):
+        m = fused.run_caustic_map(passes, p)
+        for s in (sep, single):
+            s.run(passes)
+            np.testing.assert_array_equal(m, s.caustic_map(p, which=1))
+            np.testing.assert_array_equal(fused.thickness_array(), s.thickness_array())
+            np.testing.assert_array_equal(fused.concentration_array(), s.concentration_array())
+    assert m.std() > 1e-3 * np.abs(m).max(), "the map should vary"
+
+
+def test_step_caustic_map_on_the_blocked_route(sbs, cp):
+    """The frame form, its map fused."""
+    from soap_bubble_simulation_gb300 import synthetic as S
+
+    nt, np_ = 96, 192
+    p = _vivid(cp, np_, nt)
+    sims = []
+    for _ in range(2):
+        sim = sbs.GPUDrainageSimulator(None, 500e-9, np_, nt)
+        sim.route = "blocked"
+        sim.set_thickness_array(S.smooth_modes(nt, np_, seed=3).astype(np.float32))
+        sim.enabled = True
+        sims.append(sim)
+    a, b = sims
+    for _ in range(3):
+        m_a = a.step_caustic_map(1.0 / 60.0, p)
+        b.step(1.0 / 60.0)
+        np.testing.assert_array_equal(m_a, b.caustic_map(p, which=1))
+        np.testing.assert_array_equal(a.thickness_array(), b.thickness_array())
+        assert a.current_time() == b.current_time()
