@@ -192,3 +192,70 @@ def test_resident_row_exchange_times_out_then_recovers(sbs, short_waits):
         s.run(20)
     np.testing.assert_array_equal(sims[0].thickness_array(), sims[1].thickness_array())
     np.testing.assert_array_equal(sims[0].concentration_array(), sims[1].concentration_array())
+
+
+@pytest.mark.parametrize("res,steps_per_launch", [(64, 3), (64, 2), (256, 4), (512, 3), (121, 3)])
+def test_blocked_pole_ring_exchange_times_out_then_recovers(sbs, short_waits, res, steps_per_launch):
+    """The polar strips of the blocked DrainageSimulator step (one, two and three blocks a strip) exchange
+    their ring sums; with a part that never comes the call reports the timeout, and afterwards the handle
+    steps like a fresh one, on every number of steps per launch."""
+    from soap_bubble_simulation_gb300 import synthetic
+
+    N = short_waits
+    cfg = sbs.SimulationConfig()
+    cfg.resolution = res
+    h0 = np.ascontiguousarray(synthetic.bubble_c0(res, seed=2))
+
+    def load(sim):
+        N.call("sbs_drainage_set_thickness_f64", sim.handle, N.dptr(h0), h0.size)
+
+    def field(sim):
+        out = np.empty(h0.size)
+        N.call("sbs_drainage_get_thickness_field_f64", sim.handle, N.dptr(out), out.size)
+        return out
+
+    def block(sim, k):
+        if res % 2:  # rows that are no multiple of four cells: the default K
+            sim.route = "blocked"
+        else:
+            N.call("sbs_drainage_set_time_blocking", sim.handle, k)
+        assert sim.route == "blocked"
+
+    sim, fresh = sbs.DrainageSimulator(cfg), sbs.DrainageSimulator(cfg)
+    for s in (sim, fresh):
+        block(s, steps_per_launch)
+        load(s)
+    for _ in range(2):
+        N.call("sbs_set_stall_injection", N.STALL_GRID_BARRIER)
+        with pytest.raises(sbs.SbsError) as e:
+            sim.step_n(1e-5, 4 * steps_per_launch)
+        assert e.value.code == N.SBS_E_TIMEOUT
+        N.call("sbs_set_stall_injection", 0)
+        fresh.step_n(1e-5, 4 * steps_per_launch)  # the same clock
+        for k in (steps_per_launch, 2, 3):
+            for s in (sim, fresh):
+                block(s, k)
+                load(s)
+                s.step_n(1e-5, 16)
+            np.testing.assert_array_equal(field(sim), field(fresh))
+        for s in (sim, fresh):
+            block(s, steps_per_launch)
+
+
+def test_resident_drainage_simulator_times_out_then_recovers(sbs, short_waits):
+    """The DrainageSimulator on the resident route, several rows a block."""
+    N = short_waits
+    cfg = sbs.SimulationConfig()
+    cfg.resolution = 320
+    sims = [sbs.DrainageSimulator(cfg) for _ in range(2)]
+    assert all(s.route == "resident" for s in sims)
+    N.call("sbs_set_stall_injection", N.STALL_GRID_BARRIER)
+    with pytest.raises(sbs.SbsError) as e:
+        sims[0].step_n(1e-5, 5)
+    assert e.value.code == N.SBS_E_TIMEOUT
+    N.call("sbs_set_stall_injection", 0)
+    sims[1].step_n(1e-5, 5)
+    for s in sims:
+        s.reset(500e-9)
+        s.step_n(1e-5, 30)
+    np.testing.assert_array_equal(sims[0].thickness_array(), sims[1].thickness_array())
