@@ -764,3 +764,77 @@ def test_runs_of_few_passes_match_single_steps(sbs, W, H, marangoni):
             np.testing.assert_array_equal(a, b)
         np.testing.assert_allclose(got[3], out[2][3], rtol=1e-12)
         np.testing.assert_allclose(got[4], out[2][4], rtol=1e-12)
+
+
+@pytest.mark.parametrize("marangoni", [0, 1])
+@pytest.mark.parametrize("W,H", [(9, 5), (11, 40), (119, 37), (121, 64), (122, 33), (243, 70), (1037, 131), (2051, 40),
+                                 (2177, 33), (4099, 20)])
+def test_ragged_widths_on_the_blocked_route_match_single_steps(sbs, orc, W, H, marangoni):
+    """Widths that are no multiple of four cells in the blocked kernel (the seam inside a lane's window, one
+    and several 120-column segments, a window that wraps more than once; rows of more than 2048 columns are
+    blocked by default): the bits of single steps and of the kernel-order oracle, volumes, and the fused
+    caustic map after every remainder."""
+    from soap_bubble_simulation_gb300 import synthetic
+
+    h = synthetic.smooth_modes(H, W, seed=W + H).astype(np.float32)
+    h[H // 3, : W // 4] = 25e-9  # a patch below the critical thickness
+    h[2 * H // 3, W // 2] = 1e-4  # a spike that is clamped at zero around it
+    c = synthetic.surfactant_noise(H, W, seed=H)
+    c[1, :3] = (0.0, 1.0, 0.5)
+    out = []
+    for route in ("blocked", "single"):
+        sim = sbs.GPUDrainageSimulator(None, 500e-9, W, H)
+        if W <= 2048 or route == "single":
+            sim.route = route
+        assert sim.route == route
+        sim.set_thickness_array(h)
+        sim.set_concentration_array(c)
+        sim.set_marangoni_enabled(bool(marangoni))
+        vols = sim.run_checked(0.001, 22, 11)
+        maps = [sim.run_caustic_map(n) for n in (3, 4, 6, 9, 11)]
+        out.append((sim.thickness_array(), sim.concentration_array(), vols, maps))
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+    np.testing.assert_allclose(out[0][2], out[1][2], rtol=1e-12)
+    for a, b in zip(out[0][3], out[1][3]):
+        np.testing.assert_array_equal(a, b)
+    p = orc.wgsl_params(grid_width=W, grid_height=H, marangoni_enabled=marangoni)
+    ho, co = orc.wgsl_run(p, h, c, 55, "kernel")
+    np.testing.assert_array_equal(out[0][0], ho)
+    np.testing.assert_array_equal(out[0][1], co)
+
+
+@pytest.mark.parametrize("precision", ["f32x2", "f32"])
+@pytest.mark.parametrize("res", [11, 33, 61, 121, 305, 1025])
+def test_odd_resolutions_on_the_blocked_route_match_single_steps(sbs, orc, precision, res):
+    """Odd resolutions (rows of 2 r cells, no multiple of four; pole rings of one and several blocks) in
+    the blocked kernel (1025 by default): the bits of single steps and, the smaller ones, of the
+    kernel-order oracle, fronts active (first spawn at step 50), volumes."""
+    from soap_bubble_simulation_gb300 import synthetic
+
+    h0 = synthetic.bubble_c0(res, seed=res)
+    h0[res // 3, : res // 2] = 5e-9  # below the 10 nm critical thickness: frozen
+    h0[1, : res // 3] *= 40.0
+    if precision == "f32":
+        h0 = h0.astype(np.float32).astype(np.float64)
+    dt = 0.01 if res < 1000 else 2e-5
+    out = []
+    for route in ("blocked", "single"):
+        sim = make_sim(sbs, res, precision)
+        if res < 1000 or route == "single":
+            sim.route = route
+        assert sim.route == route
+        if res >= 1000:
+            sim.step_n(0.01, 70)  # a uniform film stays stable; its clock brings the first front
+        set64(sbs, sim, h0)
+        sim.step_n(dt, 47)
+        vols = sim.run_checked(dt, 34, 17)
+        out.append((field64(sbs, sim), vols, sim.active_tfe_count()))
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_allclose(out[0][1], out[1][1], rtol=1e-12)
+    assert out[0][2] == out[1][2] >= 1
+    if res < 1000:
+        ref = orc.CpuSim(resolution=res, precision=ORC_PREC[precision])
+        ref.set_field(h0)
+        ref.step_n(dt, 81)
+        np.testing.assert_array_equal(out[0][0], ref.field())
