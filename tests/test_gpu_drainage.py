@@ -838,3 +838,38 @@ def test_odd_resolutions_on_the_blocked_route_match_single_steps(sbs, orc, preci
         ref.set_field(h0)
         ref.step_n(dt, 81)
         np.testing.assert_array_equal(out[0][0], ref.field())
+
+
+RING_EDGES = {  # words of a ring around the range of its 128-bit sums: [2^-47, 2^-16) m and 0, low words to 2^-41 m
+    "below 2^-16": np.nextafter(np.float32(2.0**-16), np.float32(0)), "2^-16": 2.0**-16,
+    "below 2^-16, low word 2^-41": float(np.nextafter(np.float32(2.0**-16), np.float32(0))) - 2.0**-41,
+    "below 2^-16, low word over it": float(np.nextafter(np.float32(2.0**-16), np.float32(0))) + 2.0**-41 - 2.0**-66,
+    "2^-47": 2.0**-47, "below 2^-47": np.nextafter(np.float32(2.0**-47), np.float32(0)), "zero": 0.0,
+    "tiny": 1e-30, "large": 5.0, "huge": 1e9}
+
+
+@pytest.mark.parametrize("route", ["resident", 2, 3, 4])
+@pytest.mark.parametrize("res", [33, 256, 512])
+def test_pole_ring_words_at_the_edges_of_the_narrow_sums(sbs, orc, res, route):
+    """Such words in the first, the last or all of the ring's column blocks (1, 2 and 3 of them in the
+    blocked kernel, one in the resident one), at either pole: the kernel-order oracle's bits."""
+    from soap_bubble_simulation_gb300 import synthetic
+
+    base = synthetic.bubble_c0(res, seed=5)
+    np_ = 2 * res
+    sim = make_sim(sbs, res, "f32x2")
+    if route == "resident" or res % 2:  # odd: blocked with the default K
+        sim.route = "resident" if route == "resident" else "blocked"
+    else:
+        set_cpu_blocking(sbs, sim, route)
+    assert sim.route == ("resident" if route == "resident" else "blocked")
+    for k, value in enumerate(RING_EDGES.values()):
+        h0 = base.copy()
+        h0[1, (3, np_ - 2, np_ // 2)[k % 3]] = value
+        h0[res - 2, (np_ - 1, slice(0, np_, 7), 0)[k % 3]] = value
+        set64(sbs, sim, h0)
+        sim.step_n(1e-9, 13)
+        ref = orc.CpuSim(resolution=res, precision=ORC_PREC["f32x2"])
+        ref.set_field(h0)
+        ref.step_n(1e-9, 13)
+        np.testing.assert_array_equal(field64(sbs, sim), ref.field())
