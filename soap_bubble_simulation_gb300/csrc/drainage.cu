@@ -298,7 +298,7 @@ int allocate(sbs_drainage *h) {
     const bool second = h->sem == SBS_WGSL_SEMANTICS || h->x2;  // the surfactant, or the low words
     const size_t o_h[2] = {piece(dev_bytes, bytes), piece(dev_bytes, bytes)};
     const size_t o_s[2] = {piece(dev_bytes, second ? bytes : 0), piece(dev_bytes, second ? bytes : 0)};
-    const size_t o_halo = piece(dev_bytes, h->resident ? resident_halo_bytes(h->rgeom, second) : 0);
+    const size_t o_halo = piece(dev_bytes, h->resident ? resident_halo_bytes(h->rgeom) : 0);
     const size_t o_part[2] = {piece(dev_bytes, sizeof(FixSum) * 2 * h->geom.nbx),
                               piece(dev_bytes, sizeof(FixSum) * 2 * h->geom.nbx)};
     const size_t o_rows = piece(dev_bytes, sizeof(float4) * h->nt), o_vol_w = piece(dev_bytes, sizeof(double) * h->nt);

@@ -257,9 +257,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) resident_kernel(const StepA
 
     // this lane's words of the row that block `of` publishes upwards (dir 0) or downwards (1) after a
     // step of parity `par`; a block of one row publishes it once
-    const int dirs = a.rb > 1 ? 2 : 1;
     auto slot = [&](int par, int of, int dir, int f) {
-        return ra.halo + ((((size_t)par * nb + of) * dirs + dir) * (TWO ? 2 : 1) + f) * (size_t)(W * 128) + col;
+        return ra.halo + ((((size_t)par * nb + of) * 2 + dir) * 2 + f) * (size_t)(W * 128) + col;
     };
     int up_dir = 0;
     if (!top) {
@@ -516,8 +515,8 @@ StepGeom resident_geometry(int nt, int np, int semantics, int x2) {
     return g;
 }
 
-size_t resident_halo_bytes(const StepGeom &g, bool two) {
-    return sizeof(unsigned long long) * 2 * g.nby * (g.rb > 1 ? 2 : 1) * (two ? 2 : 1) * (size_t)(g.wx * 128);
+size_t resident_halo_bytes(const StepGeom &g) {
+    return sizeof(unsigned long long) * 2 * g.nby * 2 * 2 * (size_t)(g.wx * 128);
 }
 
 cudaError_t launch_resident(int semantics, int x2, const StepArgs &a, const ResidentArgs &ra, const StepGeom &g,

@@ -141,7 +141,7 @@ size_t wtbc_ring_bytes(const StepGeom &g);
 cudaError_t launch_wtbc(int K, int x2, const StepArgs &a, const StepGeom &g, cudaStream_t s);
 // A chunk of steps in one launch, the field held on the chip (drainage_resident.cu): nby blocks of
 // wx warps, at most rb rows each, all resident at once. nby == 0: the grid is not supported. The
-// blocks exchange rows through resident_halo_bytes(g, two fields) of words that carry the number of their step;
+// blocks exchange rows through resident_halo_bytes(g) of words that carry the number of their step;
 // no number may come up twice while the words last, so tag0 grows by steps + 1 with every launch.
 struct ResidentArgs {
     unsigned long long *halo;
@@ -151,7 +151,7 @@ struct ResidentArgs {
     int steps;
 };
 StepGeom resident_geometry(int nt, int np, int semantics, int x2);
-size_t resident_halo_bytes(const StepGeom &g, bool two);
+size_t resident_halo_bytes(const StepGeom &g);
 cudaError_t launch_resident(int semantics, int x2, const StepArgs &a, const ResidentArgs &ra, const StepGeom &g,
                             cudaStream_t s);
 // x2: compensated f32x2 thickness (hi + lo words); CPU semantics only.
