@@ -752,6 +752,7 @@ def cpu_semantics_section(sbs, torch, h0, peak, cpu_seconds):
         sim._config = cfg
         kb = ctypes.c_int()
         N.call("sbs_drainage_time_blocking", sim.handle, ctypes.byref(kb))
+        route = sim.route  # blocked at this size; resident on grids that fit the chip
         sim.set_thickness_array(h0)
         sim.step_n(0.001, 512)
         st = torch.cuda.ExternalStream(sim.stream())
@@ -766,12 +767,14 @@ def cpu_semantics_section(sbs, torch, h0, peak, cpu_seconds):
         sim.close()
         rate = cells * n / (ms * 1e-3)
         gbs = bpc * rate / 1e9
-        out[prec] = {"value": rate, "unit": "cell-steps/s", "us_per_step": ms * 1e3 / n, "steps_per_launch": kb.value,
+        out[prec] = {"value": rate, "unit": "cell-steps/s", "us_per_step": ms * 1e3 / n, "route": route,
+                     "steps_per_launch": kb.value if route == "blocked" else 256 if route == "resident" else 1,
                      "roofline": {"bound": "hbm", "bytes_per_cell_step": bpc, "achieved": gbs, "peak": peak,
                                   "unit": "GB/s", "frac": gbs / peak,
                                   "frac_at_8B_per_cell_step": 8 * rate / 1e9 / peak,
                                   "traffic": profile_traffic("drain_wtbc_cpu_c1.md") if prec == "f32x2" else None,
-                                  "kernel": f"wtbc_kernel<{kb.value}, {'compensated' if prec == 'f32x2' else 'f32'}>"}}
+                                  "kernel": f"wtbc_kernel<{kb.value}, {'compensated' if prec == 'f32x2' else 'f32'}>"
+                                  if route == "blocked" else f"{route} route"}}
     base = cpu_baseline_f64(h0, cpu_seconds, os.cpu_count() or 1)
     out["cpu_baseline"] = base
     out["vs_cpu_baseline"] = out["f32x2"]["value"] / base["value"]
@@ -799,7 +802,7 @@ def res4096_section(sbs, synthetic, torch, peak):
     sim.close()
     rate = h.size * n / (ms * 1e-3)
     launch_us = ms * 1e3 / n * 4
-    dram = 511_542_272  # ncu DRAM bytes per 4-step launch at this size (profiles/drain_wtb_wgsl_c1.md)
+    dram = 506_536_460  # ncu DRAM bytes per 4-step launch at this size (profiles/drain_wtb_wgsl_c1.md)
     return {"value": rate, "unit": "cell-steps/s", "cells": int(h.size), "steps": n, "launch_us": launch_us,
             "roofline": {"bound": "hbm", "achieved": 16 * rate / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": 16 * rate / 1e9 / peak, "traffic": dram,

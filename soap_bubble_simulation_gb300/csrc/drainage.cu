@@ -227,11 +227,11 @@ void default_blocking(sbs_drainage *h) {
     h->wtb_k = h->cpu_k = 0;
     if (h->sem == SBS_WGSL_SEMANTICS) {
         if (!wtb_supported(h->nt, h->np)) return;
-        block_wgsl(h, 4);
+        block_wgsl(h, 4);  // K = 2, 3, 4: 2048 x 4096 13.9, 12.3, 11.8 us a pass, 4096 x 8192 50.7, 43.2, 41.3
         return;
     }
-    // steps per launch measured fastest at 2048 x 4096: 3 for the compensated storage (19.7 us
-    // per step; K = 2 20.2, K = 4 spills), 4 for plain f32 (10.7 us)
+    // us per step with K = 2, 3, 4 at 2048 x 4096: compensated storage 16.0, 14.7, 16.7 (K = 4 spills), plain
+    // f32 9.3, 8.3, 7.8; at 4096 x 8192 57.8, 53.4, 59.4 and 33.5, 29.5, 27.7
     const int k = h->x2 ? 3 : 4;
     h->cgeom = wtbc_geometry(h->nt, h->np, k, h->x2);
     if (h->cgeom.nby > 0) h->cpu_k = k;

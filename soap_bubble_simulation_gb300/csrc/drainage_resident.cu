@@ -471,8 +471,9 @@ const void *resident_fn(int sem, bool x2, bool mar, bool rag) {
 // As few rows a block as make all blocks resident at once. nby = 0: rows of more than 2048 columns,
 // or more rows than the chip holds, or, in CPU semantics, more than kCpuRows a block: from there on
 // issue decides, and the blocked step spends fewer instructions a row (640 x 1280, five rows: 4.3 us
-// here, 4.7 blocked; 768 x 1536, six: 5.1 and 4.6; the WGSL pipeline is behind at every size). Both
-// Marangoni forms of the kernel have to fit, as the choice is made per run.
+// here, 4.7 blocked; 768 x 1536, six: 5.1 and 4.6). Which WGSL runs of a grid that fits are left to the
+// other kernels all the same, resident_from() in drainage.cu says. Both Marangoni forms of the kernel have
+// to fit, as the choice is made per run.
 constexpr int kCpuRows = 5;
 static_assert(kCpuRows <= kFrontRows, "the fronts' cells of a block's rows are one word");
 StepGeom resident_geometry(int nt, int np, int semantics, int x2) {

@@ -80,9 +80,9 @@ __device__ bool grid_barrier(unsigned *bar, unsigned nblocks, unsigned extra, lo
     return *s_timeout == 0;
 }
 
-// At least three blocks per SM: the K = 4 pipeline fits 168 registers (64 bytes of spills) instead
-// of 202 (two blocks), 12 warps per SM instead of 8. Measured on the 4,096-bubble batch: 5.53e11
-// cell-steps/s against 5.35e11; four blocks (128 registers) 4.98e11.
+// At least three blocks per SM (168 registers, 12 warps). Us a step of 384, 1,024 and 4,096 bubbles at the
+// better of 32- and 64-row strips: two blocks 51.0, 124.6, 479; three 49.4, 125.0, 485; four (128 registers,
+// spills) 57.8, 145, 581.
 constexpr int kMinBlocksPerSm = 3;
 
 template <int K, bool MAR, bool RAG>

@@ -557,10 +557,10 @@ cudaError_t launch_tc(TcConvArgs a, int nf, cudaStream_t st) {
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess) return e;
     // Rows per item: the items run in rounds of as many as fit the GPU (by shared memory, 1 KB each
-    // reserved by the runtime), and the last round costs as much as a full one. Both sides as measured
-    // with three barriers a row: eight training steps of eight 256 x 512 fields took 7.6 ms with the 29
-    // (32 input channels) and 19 (16) rows this picks, 8.1 with 16 rows for all (two rounds, the second
-    // two thirds full); four 512 x 1024 fields 26.2 against 27.0, 128 x 256 2.9 against 3.3.
+    // reserved by the runtime), and the last round costs as much as a full one. Eight
+    // training steps, ms, with the rows this picks and with 16 for all: eight 256 x 512 fields (29 rows with
+    // 32 input channels, 19 with 16) 5.9, 6.4 (two rounds, the second two thirds full); four 512 x 1024 10.5,
+    // 11.5; eight 128 x 256 2.3, 2.5; one 256 x 512 1.7, 2.1.
     const long long slots = (long long)std::max(1, smem_sm / (int)(Lay::SMEM + 1024)) * sms;
     long long best = 0;
     for (int rows = 4; rows <= kTcMaxRows; ++rows) {

@@ -195,8 +195,8 @@ int ensure_ws(sbs_surrogate *s, size_t cells) {
     s->g4 = (float *)take(4 * cells);
     s->tgt = (float *)take(4 * cells);
     s->cap = cells;
-    // one loss partial per 128-cell row segment of the output layer: rows have at least 3 cells,
-    // so there are at most cells / 3 segments
+    // a loss partial per block of the output layer, which has one for every eight units of 8 columns of at
+    // least 4 rows at most: far fewer than cells / 3, also on the smallest grids
     const size_t lp = cells / 3 + 1;
     if (lp > s->loss_cap) {
         cudaFree(s->loss_part);
