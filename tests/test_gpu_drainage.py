@@ -873,3 +873,80 @@ def test_pole_ring_words_at_the_edges_of_the_narrow_sums(sbs, orc, res, route):
         ref.set_field(h0)
         ref.step_n(1e-9, 13)
         np.testing.assert_array_equal(field64(sbs, sim), ref.field())
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf, -1.0, 3e38, 1e-42])
+@pytest.mark.parametrize("marangoni", [0, 1])
+@pytest.mark.parametrize("W,H", [(132, 40), (131, 40)])
+def test_unusual_values_are_the_same_on_every_route(sbs, W, H, marangoni, bad):
+    """NaN, infinities, negative, enormous and denormal cells in either field (WGSL semantics)."""
+    from soap_bubble_simulation_gb300 import synthetic
+
+    h = synthetic.smooth_modes(H, W, seed=W).astype(np.float32)
+    c = synthetic.surfactant_noise(H, W, seed=H)
+    for k, (i, j) in enumerate([(1, 0), (H - 2, W - 1), (H // 2, W // 2), (7, 120)]):
+        (h if k % 2 else c)[i, j] = np.float32(bad)
+    h[20, 3] = np.float32(bad)
+    out = []
+    for route in ("single", "blocked", "resident"):
+        sim = sbs.GPUDrainageSimulator(None, 500e-9, W, H)
+        sim.route = route
+        sim.set_thickness_array(h)
+        sim.set_concentration_array(c)
+        sim.set_marangoni_enabled(bool(marangoni))
+        sim.run(14)
+        out.append((sim.thickness_array(), sim.concentration_array()))
+    for got in out[1:]:
+        for a, b in zip(got, out[0]):
+            np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf, -1.0, 3e38, 1e-42])
+@pytest.mark.parametrize("precision", ["f32x2", "f32"])
+@pytest.mark.parametrize("res", [66, 61])
+def test_unusual_cpu_values_are_the_same_on_every_route(sbs, res, precision, bad):
+    """The same in DrainageSimulator semantics, in a pole ring and inside, a front active."""
+    from soap_bubble_simulation_gb300 import synthetic
+
+    h0 = synthetic.bubble_c0(res, seed=res)
+    for i, j in [(1, 0), (res - 2, 2 * res - 1), (res // 2, res), (9, 119)]:
+        h0[i, j] = np.float32(bad)
+    out = []
+    for route in ("single", "blocked", "resident"):
+        sim = make_sim(sbs, res, precision)
+        sim.route = route
+        sim.step_n(0.01, 60)  # the first front
+        set64(sbs, sim, h0)
+        sim.step_n(1e-4, 13)
+        out.append(field64(sbs, sim))
+    np.testing.assert_array_equal(out[1], out[0])
+    np.testing.assert_array_equal(out[2], out[0])
+
+
+def test_handles_of_several_threads(sbs):
+    """Handles of every route stepped at once by several threads: the fields of one thread alone."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    from soap_bubble_simulation_gb300 import synthetic
+
+    jobs = [("wgsl", 64, 128, "resident"), ("wgsl", 700, 1400, "resident"), ("cpu", 128, 0, "resident"),
+            ("cpu", 256, 0, "blocked"), ("wgsl", 300, 2052, "blocked"), ("cpu", 512, 0, "resident")]
+
+    def run(job):
+        kind, nt, np_, route = job
+        if kind == "cpu":
+            sim = make_sim(sbs, nt)
+            set64(sbs, sim, synthetic.bubble_c0(nt, seed=nt))
+        else:
+            sim = sbs.GPUDrainageSimulator(None, 500e-9, np_, nt)
+            sim.set_thickness_array(synthetic.smooth_modes(nt, np_, seed=nt).astype(np.float32))
+            sim.set_dt(1e-5)
+        sim.route = route
+        for _ in range(12):
+            sim.step_n(1e-6, 70) if kind == "cpu" else sim.run(70)
+        return sim.thickness_array()
+
+    want = [run(j) for j in jobs]
+    with ThreadPoolExecutor(len(jobs)) as pool:
+        for got, w in zip(pool.map(run, jobs), want):
+            np.testing.assert_array_equal(got, w)
