@@ -271,11 +271,13 @@ int sbs_gpu_drainage_set_marangoni_params(sbs_drainage *h, float gamma_air, floa
  *                      shared memory. For grids that fit there: rows of at most
  *                      2048 columns, DrainageSimulator at most 5 rows per block.
  *  SBS_ROUTE_AUTO      what a new handle has: resident where the grid fits
- *                      (route reports that; runs of a few passes of a large grid
+ *                      (route reports that; runs of a few passes of a large grid,
+ *                      and runs while other threads' handles fill the chip too,
  *                      are launched as the blocked route does, where that is
  *                      faster), else blocked with the default K where it can
  *                      be, else single steps.
- * set_route refuses a route that the grid does not allow (SBS_E_INVALID, the
+ * FP64 volumes agree to rounding between routes (their sums are ordered by the
+ * launch's blocks). set_route refuses a route that the grid does not allow (SBS_E_INVALID, the
  * route stays). BLOCKED keeps a K chosen before. route reports the route in use
  * (never AUTO). */
 #define SBS_ROUTE_SINGLE 0

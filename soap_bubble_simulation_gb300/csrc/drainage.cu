@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -220,6 +221,13 @@ Consts &consts_of(sbs_drainage *h) { return h->k; }
 void block_wgsl(sbs_drainage *h, int K) {
     h->wtb_k = K;
     for (int mar = 0; mar < 2; ++mar) h->wgeom[mar] = wtb_geometry(h->nt, h->np, K, mar != 0);
+    h->wcrowd = wtb_crowded(h->nt, K, h->wgeom[0]);
+}
+
+// The sum of the shares of the calls in progress, per device.
+std::atomic<int> &in_progress(const sbs_drainage *h) {
+    static std::atomic<int> sums[64];
+    return sums[std::min(std::max(h->device, 0), 63)];
 }
 
 // The steps per blocked launch that a new handle has, where its grid can be blocked.
@@ -240,8 +248,17 @@ void default_blocking(sbs_drainage *h) {
 // Whether a chunk of `count` steps runs in the resident kernel. It pays the field's way into shared
 // memory and back (and the launch of resident blocks) once a chunk, so few WGSL passes of a large grid
 // are left to the other kernels (resident_from).
+//
+// Nor does it share the chip well: its blocks hold their registers while they wait. While other threads'
+// calls fill the chip as well, handles are blocked. Us a call of 256 passes (250 steps) with one, four and
+// sixteen threads, each with a handle of its own, resident, blocked and single steps or blocks as they were
+// before there was a resident kernel: 256 x 512 WGSL 331 247 247, 515 209 101, 769 206 105;
+// DrainageSimulator 512 x 1024 889 806 808, 1004 359 281, 2459 787 833. Handles that take little of the chip
+// (64 x 128) stay resident: 258 65 23, 327 95 33, 718 193 51.
 bool use_resident(const sbs_drainage *h, int count) {
-    return h->resident && count >= h->res_min[h->sem == SBS_WGSL_SEMANTICS && h->params.marangoni_enabled ? 1 : 0];
+    if (!h->resident || h->resident_always) return h->resident;
+    if (h->crowd && (h->wtb_k > 1 || h->cpu_k > 1)) return false;
+    return count >= h->res_min[h->sem == SBS_WGSL_SEMANTICS && h->params.marangoni_enabled ? 1 : 0];
 }
 
 // The fewest steps of a chunk that the resident kernel runs by default. DrainageSimulator: any number
@@ -272,6 +289,8 @@ int allocate(sbs_drainage *h) {
     h->rgeom = resident_geometry(h->nt, h->np, h->sem, h->x2);
     h->resident = h->rgeom.nby > 0;
     resident_from(h);
+    const StepGeom &sg = h->resident ? h->rgeom : h->sem == SBS_WGSL_SEMANTICS ? h->wgeom[0] : h->cgeom;
+    if (sg.cap > 0) h->share = (int)std::min<long long>(1000, 1000ll * sg.nbx * sg.nby / sg.cap);
     // one volume partial per block of whichever step kernel runs the check
     size_t vol_blocks = (size_t)h->geom.nbx * h->geom.nby;
     if (h->sem == SBS_WGSL_SEMANTICS && wtb_supported(h->nt, h->np))
@@ -529,7 +548,7 @@ int enqueue_steps(sbs_drainage *h, int start, int count, float dt, bool vol_last
         const bool cau_launch = plan[i] < 0;
         const int steps = cau_launch ? -plan[i] : plan[i];
         const int mar = h->params.marangoni_enabled ? 1 : 0;
-        const StepGeom &wg = cau_launch ? h->cau_geom[mar] : h->wgeom[mar];
+        const StepGeom &wg = cau_launch ? h->cau_geom[mar] : h->crowd ? h->wcrowd : h->wgeom[mar];
         a.rb = steps > 1 ? wg.rb : h->geom.rb;
         if (cau_launch) {
             a.cau_out = h->cau_out;
@@ -573,6 +592,7 @@ int launches_in(const sbs_drainage *h, int count, bool last_single) {
 
 // Runs one chunk (count <= kMaxChunk) through a cached CUDA graph (or directly when short).
 int run_chunk(sbs_drainage *h, int count, double dt, bool vol_last, bool last_single) {
+    h->crowd = in_progress(h) > 1000;
     const bool cpu = h->sem == SBS_CPU_SEMANTICS;
     bool use_sched = false;  // some step of the chunk has a front
     float dtf;
@@ -614,7 +634,7 @@ int run_chunk(sbs_drainage *h, int count, double dt, bool vol_last, bool last_si
         std::string key = std::to_string(h->cur) + ":" + std::to_string(count) + ":" + std::to_string(vol_last) +
                           ":" + std::to_string(use_sched) + ":" + std::to_string(bits) + ":" +
                           std::to_string(last_single) + ":" + std::to_string(h->wtb_k) + ":" +
-                          std::to_string(h->cpu_k);
+                          std::to_string(h->cpu_k) + ":" + std::to_string(h->crowd);
         if (cau_plan(h, count, last_single)) {  // the map's destination and parameters are in the graph
             uint32_t pb[4];
             std::memcpy(pb, h->cau_p, sizeof(pb));
@@ -697,6 +717,7 @@ int run_steps(sbs_drainage *h, double dt, uint64_t n, uint32_t check_every) {
 int run_with_caustics(sbs_drainage *h, uint32_t passes, const sbs_caustic_params *p, float *map, int mem) {
     const size_t bytes = sizeof(float) * (size_t)h->np * (size_t)h->nt;
     float *dst = map;
+    const DrainageInProgress now(h);
     if (mem == SBS_MEM_HOST) {
         if (!h->cau_buf) SBS_CUDA_TRY(cudaMalloc(&h->cau_buf, bytes));
         dst = h->cau_buf;
@@ -788,6 +809,8 @@ int create_common(sbs_drainage *h) {
 namespace sbs {
 int drainage_run_async(sbs_drainage *h, uint32_t passes) { return run_steps(h, 0.0, passes, 0); }
 int drainage_check(sbs_drainage *h) { return check_ring_status(h); }
+DrainageInProgress::DrainageInProgress(const sbs_drainage *h) : h_(h) { in_progress(h) += h->share; }
+DrainageInProgress::~DrainageInProgress() { in_progress(h_) -= h_->share; }
 }  // namespace sbs
 
 extern "C" {
@@ -906,6 +929,7 @@ int sbs_drainage_step_n(sbs_drainage *h, double dt, uint32_t n) {
     CHECK_HANDLE(h);
     REQUIRE_SEM(h, SBS_CPU_SEMANTICS);
     SBS_CHECK_ARG(std::isfinite(dt), "dt must be finite");
+    const DrainageInProgress now(h);
     int rc = run_steps(h, dt, n, 0);
     if (rc) return rc;
     SBS_CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -920,6 +944,7 @@ int sbs_gpu_drainage_step(sbs_drainage *h, float frame_dt) {
     const float scaled_dt = frame_dt * h->time_scale;
     const float step_dt = scaled_dt / (float)h->steps_per_frame;
     const double t0 = h->current_time;
+    const DrainageInProgress now(h);
     int rc = run_steps(h, 0.0, h->steps_per_frame, 0);
     if (rc) return rc;
     h->current_time = t0;
@@ -932,6 +957,7 @@ int sbs_gpu_drainage_run(sbs_drainage *h, uint32_t passes) {
     clear_error();
     CHECK_HANDLE(h);
     REQUIRE_SEM(h, SBS_WGSL_SEMANTICS);
+    const DrainageInProgress now(h);
     int rc = run_steps(h, 0.0, passes, 0);
     if (rc) return rc;
     SBS_CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -983,6 +1009,7 @@ int sbs_drainage_run_checked(sbs_drainage *h, double dt, uint32_t n, uint32_t ch
         SBS_CUDA_TRY(cudaMalloc(&h->vol_out, sizeof(double) * nchecks));
         h->vol_out_cap = nchecks;
     }
+    const DrainageInProgress now(h);
     SBS_CUDA_TRY(cudaMemsetAsync(h->vol_index, 0, sizeof(unsigned), h->stream));
     int rc = run_steps(h, dt, n, check_every);
     if (rc) return rc;
@@ -1353,7 +1380,7 @@ int sbs_drainage_set_route(sbs_drainage *h, int route) {
     destroy_graphs(h);
     h->resident = fits && (route == SBS_ROUTE_RESIDENT || route == SBS_ROUTE_AUTO);
     resident_from(h);
-    if (route == SBS_ROUTE_RESIDENT) h->res_min[0] = h->res_min[1] = 1;
+    h->resident_always = route == SBS_ROUTE_RESIDENT;
     return SBS_OK;
 }
 

@@ -511,6 +511,7 @@ StepGeom resident_geometry(int nt, int np, int semantics, int x2) {
         g.nbx = 1;
         g.nby = blocks;
         g.rb = rb;
+        g.cap = fit * sms;
         return g;
     }
     return g;

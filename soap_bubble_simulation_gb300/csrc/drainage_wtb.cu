@@ -203,6 +203,17 @@ StepGeom wtb_geometry(int nt, int np, int K, bool mar) {
     }
     g.nby = (nt - 2 + g.rb - 1) / g.rb;
     g.rb = (nt - 2 + g.nby - 1) / g.nby;  // evened out
+    g.cap = per_sm * sms;
+    return g;
+}
+
+// The same with strips of at least 4 K rows, for a chip that other calls fill too: what counts then is
+// the work, and short strips compute 2 K rows beside their own. 16 threads with a handle of 256 x 512
+// each, us a run of 256 passes: resident 247, blocked with its own strips 147, with these 101.
+StepGeom wtb_crowded(int nt, int K, StepGeom g) {
+    const int strips = std::max(g.cap / g.nbx, 1);
+    g.rb = std::min(std::max({(nt - 2 + strips - 1) / strips, 4 * K, g.rb}), kMaxStrip);
+    g.nby = (nt - 2 + g.rb - 1) / g.rb;
     return g;
 }
 

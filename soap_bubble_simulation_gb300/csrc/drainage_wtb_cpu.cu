@@ -690,6 +690,7 @@ StepGeom wtbc_geometry(int nt, int np, int K, int x2) {
             g.nbx = C;
             g.nby = ns;
             g.rb = rmax;
+            g.cap = per_sm * sms;
             return g;
         }
         ns = fit;

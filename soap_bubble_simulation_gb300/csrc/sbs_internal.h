@@ -60,6 +60,19 @@ cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t s);
 int drainage_run_async(sbs_drainage *h, uint32_t passes);
 int drainage_check(sbs_drainage *h);
 
+// A call that steps a handle, while it lasts: the share of the chip that the handle's launches take is
+// part of its device's sum, from which such calls see whether the chip is theirs (drainage.cu).
+class DrainageInProgress {
+  public:
+    explicit DrainageInProgress(const sbs_drainage *h);
+    ~DrainageInProgress();
+    DrainageInProgress(const DrainageInProgress &) = delete;
+    DrainageInProgress &operator=(const DrainageInProgress &) = delete;
+
+  private:
+    const sbs_drainage *h_;
+};
+
 // Area-weighted (sin theta) mean of each bubble's current thickness field of a batched foam, in
 // nm, into out[cap] (device memory); *nb = the batch's bubble count (out is written only when
 // nb <= cap). Returns when the values are there.
@@ -121,12 +134,14 @@ struct StepGeom {
     int nbx;  // column blocks
     int nby;  // row strips
     int rb;   // rows of the tallest strip
+    int cap;  // blocks that the chip holds at once (resident and blocked kernels)
 };
 
 StepGeom step_geometry(int nt, int np, int semantics, int x2);
 // Temporally blocked WGSL step (K = 2..4 steps per launch), drainage_wtb.cu.
 bool wtb_supported(int nt, int np);
 StepGeom wtb_geometry(int nt, int np, int K, bool mar);
+StepGeom wtb_crowded(int nt, int K, StepGeom g);
 cudaError_t launch_wtb(int K, const StepArgs &a, const StepGeom &g, cudaStream_t s);
 // K for a launch that also writes the caustic map of its result (a.cau_out): its final level must
 // leave one valid column beyond the kept 120 on each side of a warp's window.
@@ -259,10 +274,14 @@ struct sbs_drainage {
     sbs::StepGeom geom{};
     int wtb_k = 0;  // steps per temporally blocked launch (WGSL semantics; 0 = single steps only)
     sbs::StepGeom wgeom[2]{};          // without and with Marangoni
+    sbs::StepGeom wcrowd{};            // while other handles' calls fill the chip
     int cpu_k = 0;  // steps per temporally blocked launch (CPU semantics; 0 = single steps only)
     sbs::StepGeom cgeom{};
     bool resident = false;                     // chunks run through the resident kernel
     int res_min[2] = {1, 1};                   // of at least so many steps, without and with Marangoni
+    bool resident_always = false;              // the route was chosen by name
+    int share = 0;                             // of the chip that a launch takes, in thousandths
+    bool crowd = false;                        // the chunk under way shares the chip with other calls
     sbs::StepGeom rgeom{};
     unsigned long long *halo = nullptr;        // its row exchange
     unsigned halo_tag = 0;                     // the last step number used there

@@ -896,6 +896,7 @@ int sbs_surrogate_rollout(sbs_surrogate *s, sbs_drainage *d, uint32_t passes, ui
     SBS_CHECK_ARG(passes % SBS_NN_STEPS == 0, "passes must be a multiple of %d", SBS_NN_STEPS);
     SBS_CHECK_ARG(std::isfinite(tol) && tol > 0.0, "tol must be positive");
     SBS_CHECK_ARG(d->nt >= 4, "grid needs >= 4 theta rows");
+    const DrainageInProgress now(d);
     sbs_surrogate_stats st{};
     const size_t cells1 = (size_t)d->nt * d->np;
     if (check_every && s->scratch_cap < cells1) {

@@ -950,3 +950,40 @@ def test_handles_of_several_threads(sbs):
     with ThreadPoolExecutor(len(jobs)) as pool:
         for got, w in zip(pool.map(run, jobs), want):
             np.testing.assert_array_equal(got, w)
+
+
+@pytest.mark.parametrize("marangoni", [0, 1])
+def test_handles_that_share_the_chip(sbs, orc, marangoni):
+    """Eight threads with handles that alone fill the chip leave the resident route while they run at once:
+    the fields of one thread alone, volumes, the caustic map."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    from soap_bubble_simulation_gb300 import synthetic
+
+    sizes = [(512, 1024), (517, 1037), (300, 600), (64, 128), (900, 1801), ("cpu", 512), ("cpu", 305), (40, 2051)]
+
+    def run(size):
+        if size[0] == "cpu":
+            sim = make_sim(sbs, size[1])
+            set64(sbs, sim, synthetic.bubble_c0(size[1], seed=size[1]))
+        else:
+            nt, np_ = size
+            sim = sbs.GPUDrainageSimulator(None, 500e-9, np_, nt)
+            sim.set_thickness_array(synthetic.smooth_modes(nt, np_, seed=nt).astype(np.float32))
+            sim.set_dt(1e-5)
+            sim.set_marangoni_enabled(bool(marangoni))
+        vols, maps = [], []
+        for n in (300, 7, 64, 100, 33):
+            vols.append(sim.run_checked(1e-6, n, 25))
+            if size[0] != "cpu":
+                maps.append(sim.run_caustic_map(9))
+        return sim.thickness_array(), maps, np.concatenate(vols)
+
+    want = [run(s) for s in sizes]
+    with ThreadPoolExecutor(len(sizes)) as pool:
+        for _ in range(3):
+            for got, w in zip(pool.map(run, sizes), want):
+                np.testing.assert_array_equal(got[0], w[0])
+                for a, b in zip(got[1], w[1]):
+                    np.testing.assert_array_equal(a, b)
+                np.testing.assert_allclose(got[2], w[2], rtol=1e-12)
